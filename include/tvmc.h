@@ -221,8 +221,7 @@ typedef struct tvmc_commitment tvmc_commitment;
  *                         in 6 .. 12, else the balanced split is used); default 0 = balanced
  *   "ntt_tile_log"        log2 of the words an NTT/LDE pass CTA moves per tile (11 .. 15);
  *                         default 0 = 13
- *   "hash_unfused_tree"   1: build every Merkle level in the tree kernel instead of the lowest
- *                         eight inside the row-hash CTAs; default 0
+ *   "hash_unfused_tree"   accepted and read back; the tree kernels build every Merkle level
  *   "fail_alloc_after"    fault injection for tests: k > 0 makes the k-th device allocation the
  *                         library requests from now on fail as out-of-memory (once, on the host,
  *                         without reaching the driver); 0 disables

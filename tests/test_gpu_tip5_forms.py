@@ -1,0 +1,58 @@
+"""The two forms of the Tip5 kernels -- tensor-core (128 states per tile) and
+sixteen lanes per state -- at the edges of their tiles and of the rule between
+them, and the tensor-core LDE passes, bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import EDGE_VALUES, P, dev_empty, from_dev, rand_u64, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 127, 128, 129, 12287, 12289, 20001])
+@pytest.mark.parametrize("width", [0, 1, 9, 10, 23])
+def test_hash_rows_at_tile_edges(tv, oracle, rows, width):
+    t = rand_u64(rows * 31 + width, (max(width, 1), rows), hi=2**64 - 1)
+    t.ravel()[: EDGE_VALUES.size] = EDGE_VALUES[: t.size]
+    d, out = to_dev(t), dev_empty(rows, 5)
+    tv.hash_rows_gpu(d.data_ptr(), rows, width, out.data_ptr())
+    assert (from_dev(out) == oracle.hash_rows_cm(t[:width] % P if width else np.zeros((0, rows), np.uint64))).all()
+
+
+@pytest.mark.parametrize("n", [2, 4, 128, 256, 1 << 14, 1 << 15, 1 << 17])
+def test_merkle_levels_of_both_forms(tv, oracle, n):
+    lv = rand_u64(n, (n, 5))
+    assert (tv.merkle_heap(lv)[1:] == oracle.merkle(lv)[1:]).all()
+
+
+@pytest.mark.parametrize("count", [1, 8, 9, 8191, 8192, 20000])
+def test_pairs_and_permutations_of_both_forms(tv, oracle, count):
+    a, b = rand_u64(count, (count, 5)), rand_u64(count + 1, (count, 5))
+    got = tv.hash_pairs(a, b)
+    s = rand_u64(count + 2, (count, 16), hi=2**64 - 1)
+    perm = tv.tip5_permutations(s)
+    pick = sorted({0, 1 % count, count // 2, count - 1})
+    for i in pick:
+        assert (got[i] == oracle.hash_pair(a[i], b[i])).all()
+        assert (perm[i] == oracle.permutation(s[i] % P)).all()
+
+
+@pytest.mark.parametrize("logn", [16, 17, 18, 19, 20, 21])
+@pytest.mark.parametrize("cols,exp,offset", [(1, 4, 7), (3, 2, 3), (2, 1, 7), (1, 8, 11)])
+def test_lde_with_tensor_core_passes(tv, oracle, logn, cols, exp, offset):
+    t = rand_u64(logn * 7 + cols, (cols, 1 << logn))
+    t.ravel()[: EDGE_VALUES.size] = EDGE_VALUES % P
+    assert (tv.lde(t, exp, offset) == oracle.lde(t, exp, offset)).all()
+
+
+def test_lde_column_count_beyond_one_unit(tv, oracle):
+    """More columns than one unit of the tensor-core passes holds, and an odd count."""
+    t = rand_u64(99, (37, 1 << 20))
+    d, out = to_dev(t), dev_empty(37, 1 << 21)
+    tv.lde_gpu(d.data_ptr(), 37, 1 << 20, out.data_ptr(), 1 << 21)
+    for c in (0, 15, 16, 31, 36):
+        assert (from_dev(out[c]) == oracle.lde(t[c: c + 1], 2, 7)[0]).all()
+
+
+def test_no_wait_ran_out(tv):
+    assert tv.get_tuning("mma_timeouts") == 0

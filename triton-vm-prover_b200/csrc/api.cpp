@@ -18,6 +18,7 @@
 #include <tuple>
 #include <vector>
 
+#include "hash_mma.h"
 #include "internal.cuh"
 #include "tip5_params.h"
 #include "tvmc.h"
@@ -685,7 +686,6 @@ int tvmc::tuning_ntt_tile_log() {
     const long long v = g_tune_tile_log.load();
     return v >= 11 && v <= 15 ? (int)v : 13;
 }
-int tvmc::tuning_hash_fuse_levels() { return g_tune_unfused_tree.load() ? 0 : 8; }
 
 struct tvmc_batch {
     int device = 0;
@@ -870,6 +870,7 @@ int tvmc_get_tuning(const char* key, long long* value) {
     else if (!strcmp(key, "batch_multi_hash")) *value = g_tune_batch_multi;
     else if (!strcmp(key, "transpose_tma")) *value = g_tune_transpose_tma;
     else if (!strcmp(key, "tma_timeouts")) *value = (long long)tma_timeouts();
+    else if (!strcmp(key, "mma_timeouts")) *value = (long long)mma_timeouts();
     else if (!strcmp(key, "ntt_tile_log")) *value = g_tune_tile_log;
     else if (!strcmp(key, "fail_alloc_after")) *value = g_fail_alloc_after;
     else if (!strcmp(key, "pool_used_bytes")) {
@@ -1553,7 +1554,11 @@ int tvmc_commitment_sync(tvmc_commitment* c) {
 
 int tvmc_commitment_root(tvmc_commitment* c, uint64_t* root) {
     if (!c || !root) return fail(TVMC_ERR_INVALID, "null argument");
-    return read_sync(c, c->d_nodes + 5, 5, root);
+    uint64_t head[10];  // node 0 is zero unless a kernel of this commitment gave up waiting
+    if (int rc = read_sync(c, c->d_nodes, 10, head)) return rc;
+    if (head[0]) return fail(TVMC_ERR_TIMEOUT, "a device wait of this commitment ran out");
+    std::memcpy(root, head + 5, 40);
+    return TVMC_OK;
 }
 
 int tvmc_commitment_shape(const tvmc_commitment* c, size_t* lde_len, size_t* width) {

@@ -1,0 +1,275 @@
+// Tip5 row hashing and wide Merkle levels on the tensor-core permutation
+// (tip5_mma.cuh).
+//
+// Two threads per sponge state; a group of 256 threads takes tiles of 128 rows,
+// four groups (one CTA of 1024 threads) fill an SM, and the grid is one CTA per
+// SM: tile i goes to group (i / gridDim) mod 4 of CTA i mod gridDim, so that a
+// last, partial wave is spread over all SMs.  Rows are read column-major (a warp
+// reads 32 consecutive rows of one column, 256 contiguous bytes).  Semantics:
+// Tip5::hash_varlen (src/hash/tip5.cpp:246-282) -- zero state, overwrite the
+// rate with each full chunk and permute, last chunk = rest, 1, zeros.
+#include "hash_mma.h"
+#include "internal.cuh"
+#include "tip5_mma.cuh"
+
+namespace tvmc {
+
+namespace {
+
+extern __shared__ uint8_t t5m_smem[];
+
+__device__ __forceinline__ uint32_t dyn_base() { return (uint32_t)__cvta_generic_to_shared(t5m_smem); }
+
+// Marks a commitment whose kernels timed out: word 0 of the heap tree's unused
+// node 0 (zero otherwise).
+__device__ __forceinline__ void mark_dead(const T5Mma& c, uint64_t* heap) {
+    if (c.dead && heap) heap[0] = 1;
+}
+
+// Absorbs `perms` chunks of the row at p (element i at p[i * cs]): its n
+// elements, then 1 and zeros.  Only the chunk that holds the end tests its words.
+__device__ __forceinline__ void absorb(uint64_t (&s)[T5M_WORDS], const uint64_t* __restrict__ p, uint64_t cs,
+                                       uint32_t perms, uint32_t n, T5Mma& c) {
+    static_assert(T5M_PARTS == 2 && T5_RATE == 10, "part 0 holds rate words 0, 1, 4..9, part 1 words 2, 3");
+    const uint64_t* p0 = p + (uint64_t)(T5M_LOOKUPS * c.part) * cs;
+    const uint64_t* p1 = p + 4 * cs;
+    for (uint32_t k = 0; k < perms; k++) {
+        if ((k + 1) * T5_RATE <= n) {
+#pragma unroll
+            for (int i = 0; i < T5M_LOOKUPS; i++) s[i] = gl_to_mont(__ldg(p0 + i * cs));
+            if (c.part == 0) {
+#pragma unroll
+                for (int i = 0; i < T5_RATE - 4; i++) s[T5M_LOOKUPS + i] = gl_to_mont(__ldg(p1 + i * cs));
+            }
+            p0 += T5_RATE * cs;
+            p1 += T5_RATE * cs;
+        } else {
+#pragma unroll
+            for (int i = 0; i < T5M_WORDS; i++) {
+                const uint32_t w = t5m_word(c.part, i), j = k * T5_RATE + w;
+                if (w < T5_RATE) s[i] = j < n ? gl_to_mont(__ldg(p + (uint64_t)j * cs)) : (j == n ? T5_MONT_ONE : 0);
+            }
+        }
+        t5m_permutation(s, c);
+    }
+}
+
+__device__ __forceinline__ void zero(uint64_t (&s)[T5M_WORDS]) {
+#pragma unroll
+    for (int i = 0; i < T5M_WORDS; i++) s[i] = 0;
+}
+
+// The digest of a squeezed state: words 0-4.
+__device__ __forceinline__ void store_digest(const uint64_t (&s)[T5M_WORDS], uint64_t* p, const T5Mma& c) {
+#pragma unroll
+    for (int i = 0; i < T5M_LOOKUPS + 1; i++) {
+        const int w = t5m_word(c.part, i);
+        if (w < 5) p[w] = gl_from_mont(s[i]);
+    }
+}
+
+// hash_pair of the plain digests at l and r.
+__device__ __forceinline__ void pair_hash(uint64_t (&s)[T5M_WORDS], const uint64_t* l, const uint64_t* r, T5Mma& c) {
+#pragma unroll
+    for (int i = 0; i < T5M_WORDS; i++) {
+        const int w = t5m_word(c.part, i);
+        s[i] = w < T5_RATE ? gl_to_mont(w < 5 ? l[w] : r[w - 5]) : T5_MONT_ONE;
+    }
+    t5m_permutation(s, c);
+}
+
+// The tiles of this thread's group.
+template <class F>
+__device__ __forceinline__ void for_tiles(const T5Mma& c, uint64_t tiles, F&& body) {
+    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * c.group; t < tiles; t += (uint64_t)gridDim.x * T5M_GROUPS)
+        body(t);
+}
+
+}  // namespace
+
+// Leaf digests of `rows` rows, element (r, c) at tab[r * rstride + c * cstride]:
+// to tree leaf slots (tree non-null), else to digests.
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_mma(const uint64_t* __restrict__ tab, uint64_t rstride,
+                                                                  uint64_t cstride, uint64_t rows, uint32_t width,
+                                                                  uint64_t* __restrict__ digests,
+                                                                  uint64_t* __restrict__ tree, int layout) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    for_tiles(c, (rows + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+        const uint64_t row = tile * T5M_STATES + c.row;
+        const bool live = row < rows;
+        uint64_t s[T5M_WORDS];
+        zero(s);
+        absorb(s, tab + (live ? row : 0) * rstride, cstride, width / T5_RATE + 1, width, c);
+        if (live) store_digest(s, tree ? tree + 5 * node_slot(rows + row, rows, layout) : digests + 5 * row, c);
+    });
+    mark_dead(c, layout == LAYOUT_HEAP ? tree : nullptr);
+    t5m_done(c);
+}
+
+// The same for up to HASH_MULTI_MAX tables: tile i belongs to the job j with
+// block0[j] <= i < block0[j + 1].
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_multi_mma(const __grid_constant__ HashJobs jobs,
+                                                                        uint32_t tiles) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    for_tiles(c, tiles, [&](uint64_t tile) {
+        int j = 0;
+        for (int k = 1; k < jobs.count; k++)
+            if (jobs.j[k].block0 <= tile) j = k;
+        const uint64_t L = jobs.j[j].L;
+        const uint32_t width = jobs.j[j].width;
+        const uint64_t row = (tile - jobs.j[j].block0) * T5M_STATES + c.row;
+        const bool live = row < L;
+        uint64_t s[T5M_WORDS];
+        zero(s);
+        absorb(s, jobs.j[j].lde + (live ? row : 0), L, width / T5_RATE + 1, width, c);
+        if (live) store_digest(s, jobs.j[j].tree + 5 * (L + row), c);
+        mark_dead(c, jobs.j[j].tree);
+    });
+    t5m_done(c);
+}
+
+// Frugal streaming: absorb one stripe of `ncols` LDE columns (column-major,
+// stride L) into the sponge of every row.  Between stripes only the capacity
+// words 10..15 survive (overwrite mode replaces the rate at every absorb), so
+// they are all that is stored: cap[w*L + r], w < 6 (coalesced per word).  The
+// first stripe starts from the zero state.  Every stripe but the last must hold
+// whole 10-column chunks; the last one appends the hash_varlen padding (rest, 1,
+// zeros), finishes the digest and writes it as leaf r of the heap tree.
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_absorb_stripe_mma(const uint64_t* __restrict__ stripe, uint64_t L,
+                                                                      uint32_t ncols, uint64_t* __restrict__ cap,
+                                                                      int first, int last,
+                                                                      uint64_t* __restrict__ tree) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    for_tiles(c, (L + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+        const uint64_t row = tile * T5M_STATES + c.row;
+        const bool live = row < L;
+        uint64_t s[T5M_WORDS];
+#pragma unroll
+        for (int i = 0; i < T5M_WORDS; i++) {
+            const int w = t5m_word(c.part, i) - T5_RATE;
+            s[i] = w >= 0 && !first && live ? cap[(uint64_t)w * L + row] : 0;
+        }
+        absorb(s, stripe + (live ? row : 0), L, ncols / T5_RATE + (last ? 1 : 0), ncols, c);
+        if (!live) return;
+        if (last) {
+            store_digest(s, tree + 5 * (L + row), c);
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < T5M_WORDS; i++) {
+            const int w = t5m_word(c.part, i) - T5_RATE;
+            if (w >= 0) cap[(uint64_t)w * L + row] = s[i];
+        }
+    });
+    mark_dead(c, tree);
+    t5m_done(c);
+}
+
+// One tree level: parent p in [m/2, m) = hash_pair(node 2p, node 2p + 1).
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_level_mma(uint64_t* __restrict__ tree, uint64_t n,
+                                                                     uint64_t m, int layout) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    const uint64_t parents = m >> 1;
+    for_tiles(c, (parents + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+        const uint64_t i = tile * T5M_STATES + c.row;
+        const bool live = i < parents;
+        const uint64_t par = parents + (live ? i : 0);
+        uint64_t s[T5M_WORDS];
+        pair_hash(s, tree + 5 * node_slot(2 * par, n, layout), tree + 5 * node_slot(2 * par + 1, n, layout), c);
+        if (live) store_digest(s, tree + 5 * node_slot(par, n, layout), c);
+    });
+    mark_dead(c, layout == LAYOUT_HEAP ? tree : nullptr);
+    t5m_done(c);
+}
+
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_pairs_mma(const uint64_t* __restrict__ left,
+                                                                   const uint64_t* __restrict__ right,
+                                                                   uint64_t* __restrict__ out, uint64_t count) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    for_tiles(c, (count + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+        const uint64_t i = tile * T5M_STATES + c.row, k = i < count ? i : 0;
+        uint64_t s[T5M_WORDS];
+        pair_hash(s, left + 5 * k, right + 5 * k, c);
+        if (i < count) store_digest(s, out + 5 * i, c);
+    });
+    t5m_done(c);
+}
+
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_tip5_perm_mma(uint64_t* __restrict__ states, uint64_t count) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    for_tiles(c, (count + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+        const uint64_t i = tile * T5M_STATES + c.row;
+        const bool live = i < count;
+        uint64_t s[T5M_WORDS];
+#pragma unroll
+        for (int k = 0; k < T5M_WORDS; k++)
+            s[k] = live ? gl_to_mont(states[T5_STATE * i + t5m_word(c.part, k)]) : 0;
+        t5m_permutation(s, c);
+        if (live) {
+#pragma unroll
+            for (int k = 0; k < T5M_WORDS; k++) states[T5_STATE * i + t5m_word(c.part, k)] = gl_from_mont(s[k]);
+        }
+    });
+    t5m_done(c);
+}
+
+namespace {
+
+// One CTA per SM of the current device at most, no more than there are tiles.
+template <class... P, class... A>
+cudaError_t launch(void (*kern)(P...), uint64_t tiles, cudaStream_t st, A... args) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T5M_BYTES);
+    if (e != cudaSuccess) return e;
+    count_launch();
+    kern<<<(unsigned)(tiles < (uint64_t)sms ? tiles : (uint64_t)sms), T5M_THREADS, T5M_BYTES, st>>>(args...);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+uint64_t mma_tiles(uint64_t rows) { return (rows + T5M_STATES - 1) / T5M_STATES; }
+
+cudaError_t launch_hash_rows_mma(const uint64_t* table, uint64_t rstride, uint64_t cstride, uint64_t rows,
+                                 uint32_t width, uint64_t* digests, uint64_t* tree, int layout, cudaStream_t st) {
+    return launch(k_hash_rows_mma, mma_tiles(rows), st, table, rstride, cstride, rows, width, digests, tree, layout);
+}
+
+cudaError_t launch_hash_jobs_mma(const HashJobs& jobs, uint32_t tiles, cudaStream_t st) {
+    return launch(k_hash_rows_multi_mma, tiles, st, jobs, tiles);
+}
+
+cudaError_t launch_absorb_stripe_mma(const uint64_t* stripe, uint64_t L, uint32_t ncols, uint64_t* cap, int first,
+                                     int last, uint64_t* tree, cudaStream_t st) {
+    return launch(k_absorb_stripe_mma, mma_tiles(L), st, stripe, L, ncols, cap, first, last, tree);
+}
+
+cudaError_t launch_merkle_level_mma(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st) {
+    return launch(k_merkle_level_mma, mma_tiles(m >> 1), st, tree, n, m, layout);
+}
+
+cudaError_t launch_hash_pairs_mma(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
+                                  cudaStream_t st) {
+    return launch(k_hash_pairs_mma, mma_tiles(count), st, left, right, out, count);
+}
+
+cudaError_t launch_tip5_permutations_mma(uint64_t* states, uint64_t count, cudaStream_t st) {
+    return launch(k_tip5_perm_mma, mma_tiles(count), st, states, count);
+}
+
+unsigned int mma_timeouts() {
+    unsigned int v = 0;
+    cudaMemcpyFromSymbol(&v, g_mma8_timeouts, sizeof v);
+    return v;
+}
+
+}  // namespace tvmc

@@ -42,9 +42,6 @@ int tuning_lde_split_l1();
 // Tuning knob "ntt_tile_log": log2 of the words one NTT/LDE pass CTA moves per
 // tile (sequences per CTA = 2^(tile - log2 size), clamped); default 13.
 int tuning_ntt_tile_log();
-// Merkle levels built inside the row-hash CTA (8 by default; 0 with the tuning
-// knob "hash_unfused_tree" = 1); the rest are built by k_merkle_up.
-int tuning_hash_fuse_levels();
 
 // Merkle node storage layouts.
 //   HEAP: 2n digests, node h at h (root 1, leaves [n, 2n), slot 0 unused) --

@@ -1,4 +1,4 @@
-// Tip5 permutation for sm_100a, one sponge state per thread held in registers.
+// Tip5 round pieces for sm_100a.
 //
 // Semantics follow the reference's Tip5 (src/hash/tip5.cpp:92-203): 16-word
 // state, 5 rounds of [S-box -> MDS -> round constants].  The S-box applies
@@ -7,22 +7,14 @@
 // first column is given below.  The byte table is the offset Fermat cube map
 // x -> (x+1)^3 - 1 over F_257, generated here rather than tabulated.
 //
-// B200 layout choices (measured on sm_100a: 32-bit IMAD and DFMA are
-// half-rate, IMAD.HI quarter-rate, IMAD.WIDE takes two issue slots):
-//   * the hashing kernels keep the state in Montgomery form (w * 2^64 mod p,
-//     the representation the reference's BFieldElement holds), converting at
-//     absorb and squeeze only: the byte lookups then need no conversion, and
-//     every x^7 product reduces by a nine-instruction Montgomery reduction
-//     (gl_redc) instead of a two-step reduction and canonicalisation;
-//   * the byte table lives in shared memory as 256 words x 32 lanes, one
-//     entry per word and every lane owning its own bank, so the 8 lookups per
-//     word never conflict and the looked-up bytes are assembled by byte
-//     permutes with constant selectors;
-//   * the MDS runs exactly on the FP64 pipe (t5_mds), in parallel with the
-//     integer S-box work on the ALU/FMA pipes; being linear with integer
-//     entries it commutes with the Montgomery form, and its round constants
-//     are stored in that form;
-//   * x^7 runs unrolled over the twelve words.
+// The permutation has two forms, both on these pieces: 128 states per
+// tensor-core MDS (tip5_mma.cuh), and sixteen lanes per state (tip5_coop.cuh).
+// Both keep the state in Montgomery form (w * 2^64 mod p, the representation the
+// reference's BFieldElement holds), converting at absorb and squeeze only: the
+// byte lookups then need no conversion, every x^7 product reduces by a
+// nine-instruction Montgomery reduction (gl_redc), and the MDS, being linear with
+// integer entries, commutes with the form.  The one-thread round below, for the
+// single-round entry points, runs the MDS exactly on the FP64 pipe (t5_mds).
 #pragma once
 #include <cstdint>
 #include "field.cuh"
@@ -55,7 +47,7 @@ constexpr uint64_t t5_to_mont_const(uint64_t x) {
 // exponent bits included: each is L1 + K (H1 + K) with K = 0x43300000, which
 // adds 2K * 2^32 - K to every result; the round constants carry its negative.
 constexpr uint64_t T5_RECOMBINE_EXCESS = 2ull * 0x43300000ull * 0x100000000ull - 0x43300000ull;
-// The round constants enter in Montgomery form, like the state (t5_permutation_m).
+// The round constants enter in Montgomery form, like the state.
 struct T5RoundBias {
     double lo[T5_ROUNDS * T5_STATE];  // T5_MDS_BIAS + (rc * 2^64 mod p) & (2^32 - 1)
     double hi[T5_ROUNDS * T5_STATE];  // T5_MDS_BIAS + (rc * 2^64 mod p) >> 32
@@ -72,6 +64,17 @@ constexpr T5RoundBias t5_round_bias() {
     }
     return b;
 }
+// The round constants in Montgomery form.
+struct T5RcMont {
+    uint64_t v[T5_ROUNDS * T5_STATE];
+};
+constexpr T5RcMont t5_rc_mont() {
+    const uint64_t rc[T5_ROUNDS * T5_STATE] = {TVMC_T5_ROUND_CONSTANTS};
+    T5RcMont m{};
+    for (int i = 0; i < T5_ROUNDS * T5_STATE; i++) m.v[i] = t5_to_mont_const(rc[i]);
+    return m;
+}
+__device__ __constant__ T5RcMont c_t5_rc_mont = t5_rc_mont();
 // 1 in Montgomery form (2^64 mod p): the capacity of hash_pair and the padding 1.
 constexpr uint64_t T5_MONT_ONE = 0xFFFFFFFFull;
 __device__ __constant__ T5RoundBias c_t5_bias = t5_round_bias();
@@ -112,8 +115,7 @@ __device__ __forceinline__ uint32_t t5_lookup32(uint32_t m, const uint32_t* lane
     return __byte_perm(__byte_perm(w0, w1, 0x0040), __byte_perm(w2, w3, 0x0040), 0x5410);
 }
 
-// split_and_lookup on a state word held in Montgomery form (t5_permutation_m):
-// the reference applies the byte table to the canonical Montgomery
+// split_and_lookup on a state word held in Montgomery form: the reference applies the byte table to the canonical Montgomery
 // representation and keeps the result as the new Montgomery representation
 // (src/hash/tip5.cpp:119-145), so only a canonicalisation precedes the lookups.
 __device__ __forceinline__ uint64_t t5_split_lookup_m(uint64_t x, const uint32_t* lane_tbl) {
@@ -282,30 +284,6 @@ __device__ __forceinline__ void t5_pow7_layer_m(uint64_t s[T5_STATE]) {
     }
 }
 
-// The permutation on a state held in Montgomery form (every word w * 2^64 mod
-// p, any 64-bit representative): the form the reference's BFieldElement keeps
-// internally.  The byte lookups then need no conversion, the x^7 products
-// reduce by gl_redc, and the MDS, being linear with integer entries, commutes
-// with the form; its round constants are stored in Montgomery form.
-__device__ __forceinline__ void t5_permutation_m(uint64_t s[T5_STATE], const uint32_t* lane_tbl) {
-#pragma unroll 1
-    for (int rnd = 0; rnd < T5_ROUNDS; rnd++) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) s[i] = t5_split_lookup_m(s[i], lane_tbl);
-        t5_pow7_layer_m(s);
-        t5_mds(s, rnd);  // and the round constants
-    }
-}
-
-// The permutation on a plain state (any representatives in, canonical out).
-__device__ __forceinline__ void t5_permutation(uint64_t s[T5_STATE], const uint32_t* lane_tbl) {
-#pragma unroll
-    for (int i = 0; i < T5_STATE; i++) s[i] = gl_to_mont(s[i]);
-    t5_permutation_m(s, lane_tbl);
-#pragma unroll
-    for (int i = 0; i < T5_STATE; i++) s[i] = gl_from_mont(s[i]);
-}
-
 // One round (Tip5::round, src/hash/tip5.cpp:114-118) on a plain state, for the
 // off-path single-round and trace entry points.
 __device__ __forceinline__ void t5_round(uint64_t s[T5_STATE], const uint32_t* lane_tbl, int rnd) {
@@ -317,20 +295,6 @@ __device__ __forceinline__ void t5_round(uint64_t s[T5_STATE], const uint32_t* l
     t5_mds(s, rnd);
 #pragma unroll
     for (int i = 0; i < T5_STATE; i++) s[i] = gl_from_mont(s[i]);
-}
-
-// Tip5::hash_pair / hash_10: rate = left || right, capacity = 1s; plain digests
-// in, canonical digest out.
-__device__ __forceinline__ void t5_hash_pair(const uint64_t l[5], const uint64_t r[5], uint64_t out[5],
-                                             const uint32_t* lane_tbl) {
-    uint64_t s[T5_STATE];
-#pragma unroll
-    for (int i = 0; i < 5; i++) { s[i] = gl_to_mont(l[i]); s[5 + i] = gl_to_mont(r[i]); }
-#pragma unroll
-    for (int i = T5_RATE; i < T5_STATE; i++) s[i] = T5_MONT_ONE;
-    t5_permutation_m(s, lane_tbl);
-#pragma unroll
-    for (int i = 0; i < 5; i++) out[i] = gl_from_mont(s[i]);
 }
 
 }  // namespace tvmc
