@@ -216,7 +216,8 @@ typedef struct tvmc_commitment tvmc_commitment;
  *                         spills) or 3 (a few spills); default 3
  *   "lde_mid_variant"     1: the fused LDE middle kernel reads its twiddles from global tables per
  *                         coset; 2: it forms the inter-pass twiddles once per CTA in shared
- *                         memory for all cosets; default 2
+ *                         memory for all cosets; default 0: LDE passes of 2^8 and 2^10 points
+ *                         run on the tensor cores, others as 2
  *   "lde_split_l1"        log2 of the LDE's four-step factor n1 (6 .. 12, with log2(N) - n1 also
  *                         in 6 .. 12, else the balanced split is used); default 0 = balanced
  *   "ntt_tile_log"        log2 of the words an NTT/LDE pass CTA moves per tile (11 .. 15);

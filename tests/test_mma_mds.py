@@ -1,6 +1,6 @@
-"""The tensor-core Tip5 MDS restated on the CPU: the byte matrix, the bound on
-the 32-bit accumulators and the limb-by-limb recombination of tip5_mma.cuh
-(t5m_init, t5m_recombine) against exact integer arithmetic.  The GPU tests
+"""The tensor-core Tip5 MDS and DFTs restated on the CPU: the byte matrices, the bound on
+the 32-bit accumulators and the limb-by-limb recombination (tip5_mma.cuh,
+lde_mma.cu, mma8_recombine in mma_i8.cuh) against exact integer arithmetic.  The GPU tests
 check the same kernels through whole permutations against the oracle."""
 import os
 import random
@@ -29,7 +29,7 @@ def weights(m):
 
 
 def recombine(d):
-    """t5m_recombine on 32-bit limbs, every intermediate checked to fit."""
+    """mma8_recombine on 32-bit limbs, every intermediate checked to fit."""
     p0, p1, p2, p3 = (d[2 * i] + (d[2 * i + 1] << 8) for i in range(4))
     a = p2 + (p1 >> 16)
     assert max(p0, p1, p2, p3, a) < M32
@@ -87,3 +87,46 @@ def test_recombination_of_extreme_accumulators():
     cases = [[0] * 8, [top] * 8] + [[rng.choice((0, 1, 255, 256, top)) for _ in range(8)] for _ in range(3000)]
     for d in cases:
         assert recombine(d) == sum(x << (8 * t) for t, x in enumerate(d)) % P
+
+
+def pow2_mod(e):
+    """lde_mma.cu's 2^e (mod p), 0 <= e < 192."""
+    s = e - 96 if e >= 96 else e
+    v = 1 << s if s < 64 else (1 << (s - 32)) - (1 << (s - 64))
+    return P - v if e >= 96 else v
+
+
+def test_dft_weights_and_accumulator_bounds():
+    """B[8k + t][8j + b] = byte t of w_R^(jk) 2^(8b): exact powers of two, and no
+    accumulator or partial sum of the recombination can pass 32 bits."""
+    for R in (16, 32):
+        e1 = 78 * (32 // R)
+        assert pow(2, e1, P) == pow(7, (P - 1) // R, P)
+        worst = [0] * 8
+        for k in range(R):
+            d = [0] * 8
+            for j in range(R):
+                for b in range(8):
+                    w = pow2_mod((e1 * j * k + 8 * b) % 192)
+                    assert w < P and (w - pow(2, e1 * j * k + 8 * b, P)) % P == 0
+                    for t in range(8):
+                        d[t] += 255 * ((w >> (8 * t)) & 255)
+            worst = [max(x, y) for x, y in zip(worst, d)]
+        assert max(worst) < 2**24
+        p = [worst[2 * i] + 256 * worst[2 * i + 1] for i in range(4)]
+        assert max(p) < M32 and p[2] + (p[1] >> 16) < M32
+
+
+def test_radix_32_dft_of_bytes_is_the_dft():
+    rng = random.Random(7)
+    R = 32
+    w = pow(7, (P - 1) // R, P)
+    x = [rng.choice((0, 2**64 - 1, P, rng.randrange(2**64))) for _ in range(R)]
+    for k in (0, 1, 5, 31):
+        d = [0] * 8
+        for j in range(R):
+            for b in range(8):
+                v = pow2_mod((78 * j * k + 8 * b) % 192)
+                for t in range(8):
+                    d[t] += ((x[j] >> (8 * b)) & 255) * ((v >> (8 * t)) & 255)
+        assert recombine(d) == sum(x[j] * pow(w, j * k, P) for j in range(R)) % P

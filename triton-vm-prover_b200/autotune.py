@@ -5,7 +5,8 @@ caller's own table shapes, keeps the fastest, and persists the choice in a JSON
 cache keyed by device name and shape, so later processes start tuned:
 
     lde_mid_variant     fused LDE middle kernel: per-coset global twiddles (1) or
-                        inter-pass twiddles shared across cosets in shared memory (2)
+                        inter-pass twiddles shared across cosets in shared memory (2),
+                        or 2^8- and 2^10-point passes on the tensor cores (0)
     lde_mid_ctas        its resident CTAs/SM (2, 3)
     lde_split_l1        the LDE's four-step split N = n1 * n2 (balanced, or n1 = N^(1/2) / 4,
                         or n1 = 2^12 where valid)
@@ -77,7 +78,7 @@ def lde_candidates(log_n: int):
     splits = [0] + [l1 for l1 in (log_n // 2 - 2, 12) if 6 <= l1 <= 12 and 6 <= log_n - l1 <= 12
                     and l1 != (log_n + 1) // 2]
     return [{"lde_mid_variant": v, "lde_mid_ctas": c, "lde_split_l1": s, "ntt_tile_log": t}
-            for v in (1, 2) for c in (2, 3) for s in splits for t in (12, 13, 14)]
+            for v in (0, 1, 2) for c in (2, 3) for s in splits for t in (12, 13, 14)]
 
 
 def tune_commit(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, offset: int = 7,

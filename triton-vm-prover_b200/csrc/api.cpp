@@ -20,6 +20,7 @@
 
 #include "hash_mma.h"
 #include "internal.cuh"
+#include "lde_mma.h"
 #include "tip5_params.h"
 #include "tvmc.h"
 
@@ -676,7 +677,10 @@ std::atomic<long long> g_tune_mid_variant{0};
 // the table-sharing variant at 3 CTAs/SM was fastest (7.56 ms against 7.71 ms
 // for the per-coset variant and 8.19 ms at 2 CTAs/SM).
 int tvmc::tuning_lde_mid_ctas() { return g_tune_mid_ctas.load() == 2 ? 2 : 3; }
-int tvmc::tuning_lde_mid_variant() { return g_tune_mid_variant.load() == 1 ? 1 : 2; }
+int tvmc::tuning_lde_mid_variant() {
+    const long long v = g_tune_mid_variant.load();
+    return v == 1 || v == 2 ? (int)v : 3;
+}
 std::atomic<long long> g_tune_transpose_tma{0};
 bool tvmc::tuning_transpose_tma() { return g_tune_transpose_tma.load() == 1; }
 std::atomic<long long> g_tune_split_l1{0};
@@ -870,7 +874,7 @@ int tvmc_get_tuning(const char* key, long long* value) {
     else if (!strcmp(key, "batch_multi_hash")) *value = g_tune_batch_multi;
     else if (!strcmp(key, "transpose_tma")) *value = g_tune_transpose_tma;
     else if (!strcmp(key, "tma_timeouts")) *value = (long long)tma_timeouts();
-    else if (!strcmp(key, "mma_timeouts")) *value = (long long)mma_timeouts();
+    else if (!strcmp(key, "mma_timeouts")) *value = (long long)mma_timeouts() + lde_mma_timeouts();
     else if (!strcmp(key, "ntt_tile_log")) *value = g_tune_tile_log;
     else if (!strcmp(key, "fail_alloc_after")) *value = g_fail_alloc_after;
     else if (!strcmp(key, "pool_used_bytes")) {

@@ -33,7 +33,8 @@ int check_lde_sizes(size_t trace_len, size_t extended_len, int* logn, int* le);
 int tuning_lde_mid_ctas();
 // Tuning knob "lde_mid_variant": 1 = k_lde_mid_sym (twiddles from global tables
 // per coset), 2 = k_lde_mid_sym2 (inter-pass twiddles shared across cosets in
-// shared memory); 0 = the default (2).
+// shared memory); 0, the default, is returned as 3: passes of 2^8 and 2^10
+// points on the tensor cores (lde_mma.cu), others as 2.
 int tuning_lde_mid_variant();
 // Tuning knob "lde_split_l1": log2 of the four-step factor n1 of the LDE (the
 // K2 transform size), 0 = balanced; a split with either factor outside

@@ -36,6 +36,7 @@
 
 #include "internal.cuh"
 #include "field.cuh"
+#include "lde_mma.h"
 
 namespace tvmc {
 
@@ -885,6 +886,26 @@ static cudaError_t dispatch_ls(int l, F&& f) {
 
 static size_t words_bytes(size_t w) { return w * 8; }
 
+// Whether the tensor-core passes pay for `cols` columns of 2^l points: they take
+// one CTA per SM with tables of its own, so few short columns are better off on
+// the register networks.  B200, us (networks | tensor cores): LDE x4 of 2^14 x 16
+// 57 | 62, x 64 123 | 91, 2^15 x 16 73 | 76, x 64 201 | 173, 2^16 x 4 55 | 72, x 16 116 | 90,
+// 2^17 x 1 90 | 49, 2^18 x 1 98 | 71, 2^20 x 1 150 | 151, x 64 6080 | 4298; inverse NTT of
+// 2^14 x 64 34 | 36, x 256 92 | 79, 2^16 x 16 36 | 34, x 256 288 | 199, 2^18 x 4 34 | 42, x 16
+// 101 | 84, 2^20 x 1 44 | 57, x 4 106 | 104.
+static bool lde_mma_pays(int l, uint64_t cols) { return l >= 17 || (cols << l) >= 1ull << 20; }
+static bool ntt_mma_pays(int l, uint64_t cols) { return (cols << l) >= 3ull << 20; }
+// log2 of the four-step factor n1 that gives the tensor cores the most of a
+// 2^l-point transform: both passes where that is possible, else K2 (n1), the
+// largest part of an LDE.
+static int mma_split(int l) {
+    switch (l) {
+        case 14: case 15: case 16: case 17: return 8;
+        case 18: case 19: case 20: return 10;
+        default: return (l + 1) / 2;
+    }
+}
+
 size_t ntt_scratch_words(int logn, uint64_t cols) { return logn <= 11 ? 0 : (size_t)cols << logn; }
 
 cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t ld, uint64_t cols,
@@ -907,8 +928,10 @@ cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t 
             return cudaGetLastError();
         });
     }
-    const int l1 = (l + 1) / 2, l2 = l / 2;
+    const bool mma = ntt_mma_pays(l, cols);
+    const int l1 = mma ? mma_split(l) : (l + 1) / 2, l2 = l - l1;
     const uint64_t n = 1ull << l;
+    const uint64_t scale_mont = scale == 1 ? 0 : (uint64_t)(((unsigned __int128)scale << 64) % GL_P);
     const uint64_t* wlo = inverse ? pl.wn_i_lo : pl.wn_f_lo;
     const uint64_t* whi = inverse ? pl.wn_i_hi : pl.wn_f_hi;
     const int tile = tuning_ntt_tile_log();
@@ -917,7 +940,9 @@ cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t 
     const size_t smem_b = words_bytes((1u << l1) + spad_words(1 << l1, lTb));
     for (uint64_t c0 = 0; c0 < cols; c0 += 65535) {
         const unsigned nc = (unsigned)((cols - c0) < 65535 ? (cols - c0) : 65535);
-        cudaError_t e = dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
+        cudaError_t e = mma && lde_mma_size(l2)
+                            ? launch_pass_a_mma(l2, pl, inverse, data + c0 * ld, ld, scratch, n, nc, l1, st)
+                            : dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
             auto kern = inverse ? k_pass_a<L2, true> : k_pass_a<L2, false>;
             cudaError_t e2 = set_smem((const void*)kern, smem_a);
             if (e2 != cudaSuccess) return e2;
@@ -927,7 +952,9 @@ cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t 
             return cudaGetLastError();
         });
         if (e != cudaSuccess) return e;
-        e = dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
+        e = mma && lde_mma_size(l1)
+                ? launch_pass_b_mma(l1, pl, inverse, scratch, data + c0 * ld, ld, nc, l2, 0, scale_mont, st)
+                : dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
             auto kern = inverse ? k_pass_b<L1, true> : k_pass_b<L1, false>;
             cudaError_t e2 = set_smem((const void*)kern, smem_b);
             if (e2 != cudaSuccess) return e2;
@@ -976,7 +1003,8 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
     // "lde_split_l1" picks another valid one
     // (both factors at least 2^6, so that every pass kernel has at least one
     // whole tile of sequences)
-    int l1 = (l + 1) / 2;
+    const bool mma = tuning_lde_mid_variant() == 3 && lde_mma_pays(l, cols);
+    int l1 = mma ? mma_split(l) : (l + 1) / 2;
     if (const int ks = tuning_lde_split_l1(); ks >= 6 && ks <= 12 && l - ks >= 6 && l - ks <= 12) l1 = ks;
     // K3 holds one sequence of every coset per tile: with a large expansion a
     // smaller n2 keeps that tile within shared memory (2^22 rows x 16)
@@ -984,6 +1012,9 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
     const int l2 = l - l1;
     const int tile = tuning_ntt_tile_log();
     const uint64_t N = 1ull << l;
+    // passes of 2^8 and 2^10 points run on the tensor cores (lde_mma.cu); K2 for
+    // expansions whose per-coset tables fit and without randomizer addends
+    const bool mma_ab = mma && lde_mma_size(l2), mma_mid = mma && lde_mma_size(l1) && le <= lde_mma_max_le(l1) && !rm;
     const int lT1 = std::min(fit_lT(choose_lT(l2, tile), l2, 1), l1);
     const size_t smem1 = words_bytes((1u << l2) + spad_words(1 << l2, lT1));
     const int lT2 = std::min(fit_lT(choose_lT(l1, tile), l1, 2), l2);
@@ -995,7 +1026,8 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
         const unsigned nc = (unsigned)((cols - c0) < 65535 ? (cols - c0) : 65535);
         uint64_t* Z = scratch + (size_t)nc * N;
         const uint64_t* addc = rm ? add + c0 * ((uint64_t)rm << le) : nullptr;
-        cudaError_t e = dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
+        cudaError_t e = mma_ab ? launch_pass_a_mma(l2, pl, true, trace + c0 * tld, tld, Y, N, nc, l1, st)
+                               : dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
             cudaError_t e2 = set_smem((const void*)k_lde_inv_a<L2>, smem1);
             if (e2 != cudaSuccess) return e2;
             count_launch();
@@ -1004,10 +1036,11 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
             return cudaGetLastError();
         });
         if (e != cudaSuccess) return e;
-        e = dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
+        e = mma_mid ? launch_lde_mid_mma(l1, pl, Y, N, Z, nc, l2, hi_len, st)
+                    : dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
             if constexpr (Plan<L1>::NR == 2 && Plan<L1>::b1 == Plan<L1>::b2) {
                 constexpr int lTr = 7 - Plan<L1>::b2;
-                if (tuning_lde_mid_variant() == 2) {
+                if (tuning_lde_mid_variant() != 1) {
                     constexpr size_t R2 = (size_t)1 << Plan<L1>::b2;
                     const size_t sm2 = words_bytes(R2 * (R2 + 1) + spad_words(1 << L1, lTr) +
                                                    ((size_t)1 << (lTr + L1)) + ((size_t)1 << lTr) * (R2 + 1));
@@ -1054,7 +1087,8 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
             return cudaGetLastError();
         });
         if (e != cudaSuccess) return e;
-        e = dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
+        e = mma_ab ? launch_pass_b_mma(l2, pl, false, Z, out + c0 * old, old, nc, l1, le, 0, st)
+                   : dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
             cudaError_t e2 = set_smem((const void*)k_lde_fwd_b<L2>, smem3);
             if (e2 != cudaSuccess) return e2;
             count_launch();
