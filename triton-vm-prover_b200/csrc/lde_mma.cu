@@ -84,11 +84,32 @@ __device__ __forceinline__ uint32_t a_word(uint32_t r, uint32_t j) {
 __device__ __forceinline__ uint64_t& at64(uint8_t* p) { return *reinterpret_cast<uint64_t*>(p); }
 
 // 2^e mod p, 0 <= e < 192 (2^64 = 2^32 - 1, 2^96 = -1).
-__device__ __forceinline__ uint64_t pow2_mod(int e) {
+constexpr uint64_t pow2_mod(int e) {
     const int s = e >= 96 ? e - 96 : e;
     const uint64_t v = s < 64 ? 1ull << s : (1ull << (s - 32)) - (1ull << (s - 64));
     return e >= 96 ? GL_P - v : v;
 }
+
+// The DFT operand: word j of row n = 8 k + t, at [R n + j], holds byte t of
+// w_R^(j k) * 2^(8 b) in its byte b (w_32 = 2^78).
+template <int B>
+struct DftImage {
+    uint64_t w[LmCfg<B>::COLS * LmCfg<B>::R];
+};
+template <int B>
+constexpr DftImage<B> dft_image() {
+    constexpr int R = LmCfg<B>::R;
+    DftImage<B> im{};
+    for (int k = 0; k < R; k++)
+        for (int j = 0; j < R; j++)
+            for (int b = 0; b < 8; b++) {
+                const uint64_t v = pow2_mod((78 * (32 / R) * j * k + 8 * b) % 192);
+                for (int t = 0; t < 8; t++) im.w[R * (8 * k + t) + j] |= ((v >> (8 * t)) & 0xFF) << (8 * b);
+            }
+    return im;
+}
+static __device__ const DftImage<4> g_dft16 = dft_image<4>();
+static __device__ const DftImage<5> g_dft32 = dft_image<5>();
 
 // Every thread of the CTA calls this first.
 template <int B>
@@ -101,14 +122,12 @@ __device__ __forceinline__ void lm_init(Lm& c, const uint64_t* tw12) {
     if (tid < 32) mma8_alloc<512>(c.base + C::O_BAR + 32);
     if (tid < C::GROUPS) mma8_init_bar(c.base + C::O_BAR + 8 * tid);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    // B row n = 8 k + t, word j: byte t of w_R^(j k) * 2^(8 b), w_32 = 2^78
+    const uint64_t* img;
+    if constexpr (B == 4) img = g_dft16.w;
+    else img = g_dft32.w;
     for (int i = tid; i < C::COLS * C::R; i += LM_THREADS) {
-        const int n = i / C::R, j = i % C::R, k = n >> 3, t = n & 7;
-        uint64_t v = 0;
-#pragma unroll
-        for (int b = 0; b < 8; b++)
-            v |= ((pow2_mod((78 * (32 / C::R) * j * k + 8 * b) % 192) >> (8 * t)) & 0xFF) << (8 * b);
-        at64(c.sm + C::O_B + (j >> 4) * C::B_HALF + mma8_sw128(n, j & 15)) = v;
+        const int n = i / C::R, j = i % C::R;
+        at64(c.sm + C::O_B + (j >> 4) * C::B_HALF + mma8_sw128(n, j & 15)) = __ldg(img + i);
     }
     for (int i = tid; i < C::N; i += LM_THREADS) {
         const int d = i / C::R, k = i % C::R;

@@ -74,7 +74,6 @@ constexpr T5RcMont t5_rc_mont() {
     for (int i = 0; i < T5_ROUNDS * T5_STATE; i++) m.v[i] = t5_to_mont_const(rc[i]);
     return m;
 }
-__device__ __constant__ T5RcMont c_t5_rc_mont = t5_rc_mont();
 // 1 in Montgomery form (2^64 mod p): the capacity of hash_pair and the padding 1.
 constexpr uint64_t T5_MONT_ONE = 0xFFFFFFFFull;
 __device__ __constant__ T5RoundBias c_t5_bias = t5_round_bias();
@@ -96,6 +95,31 @@ constexpr T5Sbox t5_sbox_bytes() {
     return t;
 }
 __device__ __constant__ T5Sbox c_t5_sbox = t5_sbox_bytes();
+// The same table and the round biases of the sixteen-lane form in global memory,
+// for fills in which the threads of a warp read different entries: through the
+// constant bank those are serialised, which took most of the 9 us that a tree
+// kernel spent before its first permutation.
+static __device__ const T5Sbox g_t5_sbox = t5_sbox_bytes();
+constexpr T5RoundBias t5_coop_bias() {  // 2^52 + the constants' halves, as t5_recombine expects them
+    constexpr double centre = T5_MDS_BIAS - 4503599627370496.0;  // 2^31 * sum(M)
+    T5RoundBias b = t5_round_bias();
+    for (int i = 0; i < T5_ROUNDS * T5_STATE; i++) {
+        b.lo[i] -= centre;
+        b.hi[i] -= centre;
+    }
+    return b;
+}
+static __device__ const T5RoundBias g_t5_coop_bias = t5_coop_bias();
+struct T5MdsRow {
+    double v[2 * T5_STATE];  // the first column twice: M[(l - k) mod 16] at [l - k + 16]
+};
+constexpr T5MdsRow t5_mds_row() {
+    const double m[T5_STATE] = {TVMC_T5_MDS_FIRST_COLUMN};
+    T5MdsRow r{};
+    for (int i = 0; i < 2 * T5_STATE; i++) r.v[i] = m[i & 15];
+    return r;
+}
+static __device__ const T5MdsRow g_t5_mds_row = t5_mds_row();
 
 // Fill the lane-replicated byte table from the constant bank (all 32 lanes of
 // a warp read the same entry); call from all threads, then sync.

@@ -40,21 +40,12 @@ struct T5Coop {
 
 // Every thread of the CTA calls this once; xch: 32 entries per state of the CTA.
 __device__ __forceinline__ void t5c_init(T5Coop& c, T5CoopTables& t, double2* xch) {
-    for (int i = threadIdx.x; i < 256 * 8; i += blockDim.x) t.sbox[i] = c_t5_sbox.v[i >> 3];
-    for (int i = threadIdx.x; i < T5_ROUNDS * T5_STATE; i += blockDim.x) {
-        constexpr double centre = T5_MDS_BIAS - 4503599627370496.0;  // 2^31 * sum(M)
-        t.bias[i] = make_double2(c_t5_bias.lo[i] - centre, c_t5_bias.hi[i] - centre);
-    }
-    const double M[T5_STATE] = {TVMC_T5_MDS_FIRST_COLUMN};
+    for (int i = threadIdx.x; i < 256 * 8; i += blockDim.x) t.sbox[i] = __ldg(&g_t5_sbox.v[i >> 3]);
+    for (int i = threadIdx.x; i < T5_ROUNDS * T5_STATE; i += blockDim.x)
+        t.bias[i] = make_double2(__ldg(&g_t5_coop_bias.lo[i]), __ldg(&g_t5_coop_bias.hi[i]));
     c.lane = threadIdx.x & (T5C_LANES - 1);
 #pragma unroll
-    for (int k = 0; k < T5_STATE; k++) {  // m[k] = M[(lane - k) mod 16]
-        double v = M[0];
-#pragma unroll
-        for (int j = 1; j < T5_STATE; j++)
-            if (((c.lane - k) & 15) == j) v = M[j];
-        c.m[k] = v;
-    }
+    for (int k = 0; k < T5_STATE; k++) c.m[k] = __ldg(&g_t5_mds_row.v[c.lane - k + T5_STATE]);
     c.tbl = t.sbox + ((threadIdx.x >> 2) & 4) + (c.lane & 3);
     c.bias = t.bias + c.lane;
     c.xch = xch + (threadIdx.x / T5C_LANES) * 2 * T5_STATE;

@@ -54,9 +54,6 @@ __device__ __forceinline__ int t5m_word(int q, int i) {
     return i < T5M_LOOKUPS ? T5M_LOOKUPS * q + i : 4 + (T5M_WORDS - T5M_LOOKUPS) * q + i - T5M_LOOKUPS;
 }
 
-// The word at a position.
-__device__ __forceinline__ int t5m_at(int pos) { return t5m_word(pos / T5M_WORDS, pos % T5M_WORDS); }
-
 // Shared-memory map, as addresses in the CTA's shared window.  The byte table
 // sits on a 64 KB boundary, entry v of lane l at v * 256 + l * 4, so that one
 // byte permute of (word, lane base) is the whole address of a lookup.
@@ -71,10 +68,37 @@ constexpr uint32_t T5M_BAR = 0xA000;                   // one mbarrier per group
 constexpr uint32_t T5M_TMEM = T5M_BAR + 32;            // TMEM base address
 constexpr uint32_t T5M_BYTES = T5M_END;                // dynamic shared memory: the map from address 0
 
-struct T5MdsCol {
-    uint32_t v[T5_STATE];
+// The constant operand images: B (word w of row n at [16 n + w], by position) and
+// byte t of word r's round constants, in Montgomery form, at [round][8 r + t].
+struct T5mImages {
+    uint64_t b[T5M_STATES * T5_STATE];
+    uint32_t rc[T5_ROUNDS * T5M_STATES];
 };
-__device__ __constant__ T5MdsCol c_t5_mds_col = {{TVMC_T5_MDS_FIRST_COLUMN}};
+constexpr int t5m_at_const(int pos) {
+    const int q = pos / T5M_WORDS, i = pos % T5M_WORDS;
+    return i < T5M_LOOKUPS ? T5M_LOOKUPS * q + i : 4 + (T5M_WORDS - T5M_LOOKUPS) * q + i - T5M_LOOKUPS;
+}
+constexpr T5mImages t5m_images() {
+    const uint64_t col[T5_STATE] = {TVMC_T5_MDS_FIRST_COLUMN};
+    const T5RcMont rc = t5_rc_mont();
+    T5mImages im{};
+    for (int n = 0; n < T5M_STATES; n++) {
+        const int r = t5m_at_const(n >> 3), t = n & 7;
+        for (int w = 0; w < T5_STATE; w++) {
+            const uint64_t m = col[(r - t5m_at_const(w)) & 15];
+            uint64_t v = 0;
+            for (int b = 0; b < 8; b++) {
+                const uint64_t x = b < 7 ? m << (8 * b) : (m << 56) + (m >> 8) * 0xFFFFFFFFull;
+                v |= ((x >> (8 * t)) & 0xFF) << (8 * b);
+            }
+            im.b[16 * n + w] = v;
+        }
+        for (int rnd = 0; rnd < T5_ROUNDS; rnd++)
+            im.rc[T5M_STATES * rnd + n] = (uint32_t)(rc.v[rnd * T5_STATE + r] >> (8 * t)) & 0xFF;
+    }
+    return im;
+}
+static __device__ const T5mImages g_t5m_images = t5m_images();
 
 // What a thread keeps of its group's MMA.
 struct T5Mma {
@@ -153,32 +177,19 @@ __device__ __forceinline__ uint64_t t5m_pow7(uint64_t x) {
 __device__ __forceinline__ void t5m_init(T5Mma& c, uint32_t dyn) {
     c.base = (dyn + 1023) & ~1023u;
     const int tid = threadIdx.x;
-    auto st8 = [](uint32_t a, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); };
     if (tid < 32) mma8_alloc<T5M_COLS>(c.base + T5M_TMEM);
     if (tid < T5M_GROUPS) mma8_init_bar(c.base + T5M_BAR + 8 * tid);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int i = tid; i < T5_SBOX_WORDS; i += T5M_THREADS)
-        sts32(T5M_SBOX + (i >> 5) * 256 + (i & 31) * 4, c_t5_sbox.v[i >> 5]);
-    // ones and round-constant tiles: zero, then byte k = 0 of every row
-    for (int i = tid; i < 6 * 1024; i += T5M_THREADS) sts32(c.base + T5M_ONES + 4 * i, 0);
-    for (int i = tid; i < T5M_STATES * T5_STATE; i += T5M_THREADS) {  // B row n, word c
-        const int n = i >> 4, w = i & 15, t = n & 7;  // w: position of the input word
-        const uint64_t m = c_t5_mds_col.v[(t5m_at(n >> 3) - t5m_at(w)) & 15];
-        uint64_t v = 0;
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            const uint64_t x = b < 7 ? m << (8 * b) : (m << 56) + (m >> 8) * 0xFFFFFFFFull;
-            v |= ((x >> (8 * t)) & 0xFF) << (8 * b);
-        }
-        sts64(c.base + T5M_B + mma8_sw128(n, w), v);
+        sts32(T5M_SBOX + (i >> 5) * 256 + (i & 31) * 4, __ldg(&g_t5_sbox.v[i >> 5]));
+    // ones and round-constant tiles: byte k = 0 of every row, zero elsewhere
+    for (int i = tid; i < 6 * 256; i += T5M_THREADS) {  // 16-byte chunk j of row n of a tile
+        const int tile = i >> 8, n = (i >> 1) & 127, j = i & 1;
+        const uint32_t v = j ? 0u : (tile == 0 ? 1u : __ldg(&g_t5m_images.rc[T5M_STATES * (tile - 1) + n]));
+        sts128(c.base + T5M_ONES + tile * 4096 + (n >> 3) * 256 + j * 128 + (n & 7) * 16, v, 0);
     }
-    __syncthreads();
-    for (int i = tid; i < 6 * 128; i += T5M_THREADS) {
-        const int tile = i >> 7, n = i & 127;
-        const uint32_t v = tile == 0 ? 1u
-                                     : (uint32_t)(c_t5_rc_mont.v[(tile - 1) * T5_STATE + t5m_at(n >> 3)] >> (8 * (n & 7))) & 0xFF;
-        st8(c.base + T5M_ONES + tile * 4096 + (n >> 3) * 256 + (n & 7) * 16, v);
-    }
+    for (int i = tid; i < T5M_STATES * T5_STATE; i += T5M_THREADS)
+        sts64(c.base + T5M_B + mma8_sw128(i >> 4, i & 15), __ldg(&g_t5m_images.b[i]));
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
