@@ -157,6 +157,9 @@ size_t lde_scratch_words(int logn, int log_exp, uint64_t cols);
 cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, uint64_t* out, uint64_t old,
                        uint64_t cols, uint64_t* scratch, cudaStream_t st, const uint64_t* add = nullptr,
                        int rm = 0);
+// The same for trace lengths 2^1 .. 2^11: whole columns per CTA, no scratch.
+cudaError_t launch_lde_small(const LdePlan& pl, const uint64_t* trace, uint64_t tld, uint64_t* out, uint64_t old,
+                             uint64_t cols, const uint64_t* add, int rm, cudaStream_t st);
 // Interpolant coefficients touched by R randomizer coefficients: min(N, R).
 inline int rand_rows(int logn, uint64_t R) {
     return R < (1ull << logn) ? (int)R : (1 << logn);
