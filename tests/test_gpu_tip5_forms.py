@@ -54,5 +54,29 @@ def test_lde_column_count_beyond_one_unit(tv, oracle):
         assert (from_dev(out[c]) == oracle.lde(t[c: c + 1], 2, 7)[0]).all()
 
 
+@pytest.mark.parametrize("logn,cols,R,exp", [(12, 256, 98, 4), (16, 16, 5, 2), (17, 2, 300, 4), (20, 1, 98, 4), (18, 2, 1, 8)])
+def test_randomized_lde_with_tensor_core_passes(tv, oracle, logn, cols, R, exp):
+    t, r = rand_u64(logn + cols, (cols, 1 << logn)), rand_u64(logn + R, (cols, R))
+    got = tv.lde_randomized(t, r, exp, 7, 3)
+    for c in sorted({0, cols // 2, cols - 1}):
+        assert (got[c] == oracle.lde_randomized(t[c: c + 1], r[c: c + 1], exp, 7, 3)[0]).all()
+
+
+@pytest.mark.parametrize("logn,cols", [(1, 300), (5, 33), (6, 5), (8, 379), (9, 3), (11, 2)])
+@pytest.mark.parametrize("exp", [1, 2, 8, 16])
+def test_short_columns_with_any_number_of_cosets(tv, oracle, logn, cols, exp):
+    t = rand_u64(logn * cols + exp, (cols, 1 << logn))
+    assert (tv.lde(t, exp, 7) == oracle.lde(t, exp, 7)).all()
+
+
+@pytest.mark.parametrize("logn,cols", [(12, 800), (13, 400), (16, 48), (18, 13), (20, 3), (21, 2)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_ntt_with_tensor_core_passes(tv, oracle, logn, cols, inverse):
+    a = rand_u64(logn + cols, (cols, 1 << logn), hi=2**64 - 1)
+    got = tv.ntt(a, inverse=inverse)
+    for c in sorted({0, cols // 2, cols - 1}):
+        assert (got[c] == oracle.ntt(a[c] % P, inverse=inverse)).all()
+
+
 def test_no_wait_ran_out(tv):
     assert tv.get_tuning("mma_timeouts") == 0

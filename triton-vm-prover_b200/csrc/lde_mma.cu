@@ -1,30 +1,32 @@
-// LDE passes with 2^10-point sub-transforms on the integer tensor cores.
+// LDE and NTT passes with 2^8- or 2^10-point sub-transforms on the integer
+// tensor cores.
 //
-// A 2^10-point sub-transform is two rounds of radix 32 (ntt.cu, sub_dft).  A
-// radix-32 DFT over the field is a constant 32 x 32 map, so here it is an exact
-// byte GEMM (mma_i8.cuh): 128 lines of 32 words form A (128 x 256 bytes), the
-// DFT matrix B is 256 x 256 bytes (64 KB, filled once per CTA), and D is
-// 128 x 256 in TMEM.  A radix-32 register network costs about 55 instructions
-// per element (80 butterflies of two additions and a shift-twiddle over 32
-// elements); the MMA form leaves the recombination of eight 32-bit
-// accumulators, 17, and takes inputs of any representative, so that nothing is
-// canonicalised on the way in.  The tensor pipe needs 1024 cycles per 4096
-// elements and round, about a third of what the twiddle products and the
-// recombination take.
+// A sub-transform of N = R * R points, R = 16 or 32, is two rounds of radix R
+// (ntt.cu, sub_dft).  A radix-R DFT over the field is a constant R x R map, so
+// here it is an exact byte GEMM (mma_i8.cuh): 128 lines of R words form A
+// (128 x 8 R bytes), the DFT matrix B is 8 R x 8 R bytes (16 or 64 KB, copied in
+// once per CTA), and D is 128 x 8 R in TMEM.  A radix-32 register network costs
+// about 55 instructions per element (80 butterflies of an addition and a
+// shift-twiddled subtraction over 32 elements); the MMA form leaves the
+// recombination of eight 32-bit accumulators, 17, and takes inputs of any
+// representative, so that nothing is canonicalised on the way in.  The tensor
+// pipe needs 1024 cycles per 4096 elements and round at R = 32 (256 per 2048 at
+// R = 16), about a third of what the twiddle products and the recombination take.
 //
-// A group of 512 threads owns a tile of four sequences of 1024 elements (128
-// lines), its A tile and 256 TMEM columns; the two groups of a CTA (one CTA per
-// SM) work on different columns or blocks, so that one computes while the
-// other waits for its MMA.  TMEM lane = line; four threads share a line, part q
-// holding outputs 8 q .. 8 q + 7.  The A tile is also the transpose buffer
-// between the two rounds: lines are ordered t + 4 * d (t: sequence, d: digit),
-// so that the final global accesses come in runs of four words (one 32-byte
-// sector), except where a sequence is contiguous in memory (d + 32 * t).
+// A group of 512 (R = 32) or 256 threads owns a tile of 128 lines (4 or 8
+// sequences), its A tile and 8 R TMEM columns; the two or four groups of a CTA
+// (one CTA per SM) work on different columns or tiles, so that the others compute
+// while one waits for its MMA.  TMEM lane = line; R / 8 threads share a line, part
+// q holding outputs 8 q .. 8 q + 7.  The A tile is also the transpose buffer
+// between the two rounds: lines are ordered t + SEQS * d (t: sequence, d: digit),
+// so that the final global accesses come in runs of SEQS words (one or two
+// 32-byte sectors), except where a sequence is contiguous in memory (d + R * t).
 //
-// B200: LDE x4 of 32 x 2^20 3.04 -> 2.00 ms, 256 x 2^18 7.15 -> 3.57, 256 x 2^16 1.31 -> 0.85;
-// D read 16 columns at a time (32 at a time: 2.03 against 1.95 ms).  What bounds
+// B200: LDE x4 of 32 x 2^20 3.04 -> 1.97 ms, 256 x 2^18 7.15 -> 3.57, 256 x 2^16 1.31 -> 0.85.
+// D is read 16 columns at a time (32 at a time: 2.03 against 1.95 ms), the next 16
+// while the current ones are recombined (128 x 2^16 0.453 -> 0.431 ms).  What bounds
 // it: the twiddle products and recombinations on the integer pipes (60% and 40%
-// busy) and the MMA's latency, which one other group covers only in part.
+// busy) and the MMA's latency, which the other groups cover only in part.
 #include "lde_mma.h"
 #include "mma_i8.cuh"
 
@@ -173,12 +175,14 @@ __device__ __forceinline__ void lm_dft(Lm& c, F&& out) {
         mma8_commit(c.bar);
     }
     mma8_wait(c.bar, c.phase, c.dead);
+    uint32_t d[2][16];
+    mma8_ld16(d[0], c.tmem);
 #pragma unroll
     for (int h = 0; h < 4; h++) {
-        uint32_t d[16];
-        mma8_ld16(d, c.tmem + 16 * h);
+        mma8_ld_wait(d[h & 1]);
+        if (h < 3) mma8_ld16(d[(h + 1) & 1], c.tmem + 16 * (h + 1));
 #pragma unroll
-        for (int i = 0; i < 2; i++) out(2 * h + i, mma8_recombine(d + 8 * i));
+        for (int i = 0; i < 2; i++) out(2 * h + i, mma8_recombine(d[h & 1] + 8 * i));
     }
 }
 
@@ -294,14 +298,16 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_pass_a_mma(const uint64_t* __
 // N^-1 s_c^i, forward DFT, times w_N^(k2 q) -> Z_c[k2 + n2*q], n2 = 2^l2.  The
 // coset scale is applied as in k_lde_mid_sym2: s_c^(n2*ln) rides on the first
 // round's output twiddle (one table per coset), the rest is one product with a
-// table entry per (row, k1) of the block.
-template <int B>
+// table entry per (row, k1) of the block.  RAND: the raw coefficients i < rm get
+// the addends of launch_rand_addend first.
+template <int B, bool RAND>
 __global__ void __launch_bounds__(LM_THREADS, 1) k_lde_mid_mma(const uint64_t* __restrict__ Y, uint64_t yld,
                                                                uint64_t* __restrict__ Z, uint32_t cols, uint32_t unit,
                                                                int l2, int le,
                                                                const uint64_t* tw12, const uint64_t* wlo,
                                                                const uint64_t* whi, const uint64_t* sc_lo,
-                                                               const uint64_t* sc_hi, int hi_len) {
+                                                               const uint64_t* sc_hi, int hi_len,
+                                                               const uint64_t* __restrict__ add, int rm) {
     using C = LmCfg<B>;
     Lm c;
     lm_init<B>(c, tw12);
@@ -344,7 +350,14 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_lde_mid_mma(const uint64_t* _
                 const uint64_t* sc = reinterpret_cast<const uint64_t*>(scl + e * C::SCL_BYTES) + t * C::TWP + 8 * c.part;
                 uint64_t v[8];
 #pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = gl_mont_mul(cf[i], sc[i]);
+                for (int i = 0; i < 8; i++) {
+                    uint64_t x = cf[i];
+                    if constexpr (RAND) {  // addends of the first rm coefficients
+                        const uint32_t ci = ((uint32_t)(C::R * (8 * c.part + i) + d) << l2) + k20 + t;
+                        if (ci < (uint32_t)rm) x = gl_add_pc(x, add[((uint64_t)col * E + e) * rm + ci]);
+                    }
+                    v[i] = gl_mont_mul(x, sc[i]);
+                }
                 lm_fill<B>(c, v);
                 lm_round1<B>(c, t, d, twc + e * C::TWC_BYTES);
                 lm_store<B>(c, dst, l2, [&](int i, uint64_t x) { return gl_mont_mul(x, twq[128 * i]); });
@@ -430,12 +443,13 @@ cudaError_t pass_a(const LdePlan& pl, bool inverse, const uint64_t* in, uint64_t
 }
 template <int B>
 cudaError_t mid(const LdePlan& pl, const uint64_t* Y, uint64_t yld, uint64_t* Z, uint32_t cols, int l2, int hi_len,
-                cudaStream_t st) {
+                const uint64_t* add, int rm, cudaStream_t st) {
     using C = LmCfg<B>;
     const uint64_t blocks = (1u << l2) / C::SEQS;
     const uint32_t unit = unit_cols<B>(blocks, cols);
-    return launch(k_lde_mid_mma<B>, blocks * ((cols + unit - 1) / unit), C::mid_bytes(pl.log_exp), st, Y, yld, Z, cols,
-                  unit, l2, pl.log_exp, pl.tw12_f, pl.wn_f_lo, pl.wn_f_hi, pl.sc_lo, pl.sc_hi, hi_len);
+    return launch(rm ? k_lde_mid_mma<B, true> : k_lde_mid_mma<B, false>, blocks * ((cols + unit - 1) / unit),
+                  C::mid_bytes(pl.log_exp), st, Y, yld, Z, cols, unit, l2, pl.log_exp, pl.tw12_f, pl.wn_f_lo,
+                  pl.wn_f_hi, pl.sc_lo, pl.sc_hi, hi_len, add, rm);
 }
 template <int B>
 cudaError_t pass_b(const LdePlan& pl, bool inverse, const uint64_t* Z, uint64_t* out, uint64_t old, uint32_t cols,
@@ -455,8 +469,9 @@ cudaError_t launch_pass_a_mma(int lsub, const LdePlan& pl, bool inverse, const u
 }
 
 cudaError_t launch_lde_mid_mma(int lsub, const LdePlan& pl, const uint64_t* Y, uint64_t yld, uint64_t* Z, uint32_t cols,
-                               int l2, int hi_len, cudaStream_t st) {
-    return lsub == 10 ? mid<5>(pl, Y, yld, Z, cols, l2, hi_len, st) : mid<4>(pl, Y, yld, Z, cols, l2, hi_len, st);
+                               int l2, int hi_len, const uint64_t* add, int rm, cudaStream_t st) {
+    return lsub == 10 ? mid<5>(pl, Y, yld, Z, cols, l2, hi_len, add, rm, st)
+                      : mid<4>(pl, Y, yld, Z, cols, l2, hi_len, add, rm, st);
 }
 
 cudaError_t launch_pass_b_mma(int lsub, const LdePlan& pl, bool inverse, const uint64_t* Z, uint64_t* out, uint64_t old,

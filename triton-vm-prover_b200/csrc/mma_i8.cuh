@@ -135,12 +135,14 @@ __device__ __forceinline__ void mma8_ld32(uint32_t (&d)[32], uint32_t a) {
         : "r"(a));
     asm volatile("tcgen05.wait::ld.sync.aligned;" : TVMC_RW8(0), TVMC_RW8(8), TVMC_RW8(16), TVMC_RW8(24)::"memory");
 }
-__device__ __forceinline__ void mma8_ld16(uint32_t* d, uint32_t a) {
+__device__ __forceinline__ void mma8_ld16(uint32_t (&d)[16], uint32_t a) {  // valid after mma8_ld_wait
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
         "%15}, [%16];"
         : TVMC_W8(0), TVMC_W8(8)
         : "r"(a));
+}
+__device__ __forceinline__ void mma8_ld_wait(uint32_t (&d)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : TVMC_RW8(0), TVMC_RW8(8)::"memory");
 }
 #undef TVMC_W8

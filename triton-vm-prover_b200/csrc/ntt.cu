@@ -724,8 +724,8 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
     const int tile = tuning_ntt_tile_log();
     const uint64_t N = 1ull << l;
     // passes of 2^8 and 2^10 points run on the tensor cores (lde_mma.cu); K2 for
-    // expansions whose per-coset tables fit and without randomizer addends
-    const bool mma_ab = mma && lde_mma_size(l2), mma_mid = mma && lde_mma_size(l1) && le <= lde_mma_max_le(l1) && !rm;
+    // expansions whose per-coset tables fit
+    const bool mma_ab = mma && lde_mma_size(l2), mma_mid = mma && lde_mma_size(l1) && le <= lde_mma_max_le(l1);
     const int lT1 = std::min(fit_lT(choose_lT(l2, tile), l2, 1), l1);
     const size_t smem1 = words_bytes((1u << l2) + spad_words(1 << l2, lT1));
     const int lT2 = std::min(fit_lT(choose_lT(l1, tile), l1, 2), l2);
@@ -747,7 +747,7 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
             return cudaGetLastError();
         });
         if (e != cudaSuccess) return e;
-        e = mma_mid ? launch_lde_mid_mma(l1, pl, Y, N, Z, nc, l2, hi_len, st)
+        e = mma_mid ? launch_lde_mid_mma(l1, pl, Y, N, Z, nc, l2, hi_len, addc, rm, st)
                     : dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
             if constexpr (Plan<L1>::NR == 2 && Plan<L1>::b1 == Plan<L1>::b2) {
                 constexpr int lTr = 7 - Plan<L1>::b2;
