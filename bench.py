@@ -660,7 +660,7 @@ def run_ours(args):
                        "tuning": tuned.get("knobs", {}), "tuning_s": tuned.get("seconds", {}),
                        "streams": args.streams,
                        "parallelism": "replicas" if ws > 1 else "1 gpu"},
-            "roofline": {"bound": "int32", "kernel": "k_hash_rows + k_merkle_level + k_merkle_up (Tip5)",
+            "roofline": {"bound": "int32", "kernel": "k_hash_rows_mma + k_merkle_level_mma + k_merkle_coop (Tip5)",
                          "achieved": achieved_int, "peak": int_peak, "unit": "Top/s",
                          "frac": achieved_int / int_peak,
                          "peak_source": f"SM issue limit: {sms} SMs x {ISSUE_LANES_PER_SM} lanes x {sm_mhz:.0f} MHz "
