@@ -227,7 +227,8 @@ typedef struct tvmc_commitment tvmc_commitment;
  *                         library requests from now on fail as out-of-memory (once, on the host,
  *                         without reaching the driver); 0 disables
  * Unknown keys return TVMC_ERR_INVALID.  tvmc_get_tuning also reads "pool_used_bytes": the bytes
- * currently allocated from the current device's stream-ordered pool (a leak check). */
+ * currently allocated from the current device's stream-ordered pool (a leak check), and
+ * "mma_timeouts": tensor-core waits that gave up (after about a second; 0 unless a GPU fails). */
 int tvmc_set_tuning(const char* key, long long value);
 /* The library keeps its LDE/NTT scratch, upload staging and the LDE of
  * TVMC_DISCARD_LDE commitments per (device, stream) once used, and the device's
@@ -310,7 +311,8 @@ int tvmc_sponge_absorb_gpu(uint64_t* d_state, const uint64_t* d_data, size_t len
  * (discriminant 0, then the 5 root words), into d_state on `stream`, ordered
  * after the commitment: the root never visits the host (src/gpu/gpu_stark.cu:2577-2585). */
 int tvmc_commitment_absorb_root(tvmc_commitment* c, uint64_t* d_state, void* stream);
-/* Wait for the commitment and copy its root (5 words) to host memory. */
+/* Wait for the commitment and copy its root (5 words) to host memory; TVMC_ERR_TIMEOUT if one of its
+ * hash kernels gave up waiting. */
 int tvmc_commitment_root(tvmc_commitment* c, uint64_t* root);
 int tvmc_commitment_sync(tvmc_commitment* c);
 /* Sizes: LDE length (= number of leaves) and width. */
