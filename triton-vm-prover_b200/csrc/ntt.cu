@@ -41,6 +41,10 @@
 
 namespace tvmc {
 
+// The forward 32-point root as a power of two, as the register networks apply it.
+constexpr int GL_W32_LOG2 = 78;
+static_assert(GL_W32_LOG2 == W32_LOG2, "the networks of ntt_sub.cuh use this root");
+
 // ---------------------------------------------------------------- plain NTT
 
 // Whole columns per CTA: T = 2^lT columns, size 2^LS <= 2^11, in place.  All

@@ -44,7 +44,7 @@ __device__ __forceinline__ constexpr int brevc(int k) {
 
 // The forward 32-point root w_32 = 7^((p-1)/32) is 2^78 (mod p); every root of
 // order 2^m <= 32 is its power 2^(78 * 2^(5-m) mod 192).
-constexpr int GL_W32_LOG2 = 78;
+constexpr int W32_LOG2 = 78;
 
 // Radix-2 DIF network on R = 2^B registers (forward root); X[k] ends in
 // v[brev(k)].  Its twiddles w_{2h}^j are roots of order <= 32, applied as
@@ -63,7 +63,7 @@ __device__ __forceinline__ void reg_dft(uint64_t (&v)[1 << B]) {
             for (int j = 0; j < h; j++) {
                 const uint64_t a = v[blk + j], c = v[blk + j + h];
                 v[blk + j] = gl_add_c(a, c);
-                v[blk + j + h] = gl_sub_mul_pow2_c(a, c, (GL_W32_LOG2 * j * (16 / h)) % 192);
+                v[blk + j + h] = gl_sub_mul_pow2_c(a, c, (W32_LOG2 * j * (16 / h)) % 192);
             }
         }
     }
