@@ -252,7 +252,12 @@ def run_reference(args):
     if rank != 0:
         return
     from oracle import RefLib
-    r = RefLib()
+    try:
+        r = RefLib()
+    except FileNotFoundError as e:
+        print(json.dumps({"impl": "reference",
+                          "unavailable": f"{e} not built (make -C oracle ref needs the reference tree)"}))
+        return
     cores = r.max_threads()
     n = 1 << args.log_n
     L = EXPANSION * n
@@ -643,9 +648,12 @@ def run_ours(args):
 
     cpu = None
     if rank == 0 and ws == 1 and not args.skip_cpu:
-        v, cores, sample, detail = cpu_reference_sample(args.log_n)
-        cpu = {"value": v, "unit": "cells/s", "cores": cores, "kind": "reference", "sample": sample,
-               "est_commit_s": detail["est_commit_s"], "extrapolated": True, "cpu_model": cpu_model()}
+        try:
+            v, cores, sample, detail = cpu_reference_sample(args.log_n)
+            cpu = {"value": v, "unit": "cells/s", "cores": cores, "kind": "reference", "sample": sample,
+                   "est_commit_s": detail["est_commit_s"], "extrapolated": True, "cpu_model": cpu_model()}
+        except FileNotFoundError as e:
+            cpu = {"unavailable": f"{e} not built (make -C oracle ref needs the reference tree)"}
 
     if rank == 0:
         line = {
