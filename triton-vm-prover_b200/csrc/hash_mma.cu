@@ -227,8 +227,7 @@ cudaError_t launch(void (*kern)(P...), uint64_t tiles, cudaStream_t st, A... arg
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T5M_BYTES);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)kern);
     if (e != cudaSuccess) return e;
     count_launch();
     kern<<<(unsigned)(tiles < (uint64_t)sms ? tiles : (uint64_t)sms), T5M_THREADS, T5M_BYTES, st>>>(args...);

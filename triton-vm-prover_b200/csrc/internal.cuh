@@ -19,6 +19,14 @@ struct NvtxRange {
     NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Lets fn, a kernel without static shared memory, take all of an SM's dynamic
+// shared memory.  The limit is a property of the function, shared by every
+// thread of the process, and each launch states its own size: so it is only ever
+// set to this one value.  Set to each call's own size, it let one thread lower it
+// between another's call and launch, which then failed as an invalid value.
+inline cudaError_t raise_smem_limit(const void* fn) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
 // Number of kernels this library has launched (all devices, all threads).
 void count_launch();
 // Records `msg` as the calling thread's tvmc_last_error() text; returns code.

@@ -413,8 +413,7 @@ int sm_count() {
 // At most one CTA per SM.
 template <class... P, class... A>
 cudaError_t launch(void (*kern)(P...), uint64_t work, uint32_t bytes, cudaStream_t st, A... args) {
-    const cudaError_t e =
-        cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes + LM_SLACK));
+    const cudaError_t e = raise_smem_limit((const void*)kern);
     if (e != cudaSuccess) return e;
     const uint64_t sms = (uint64_t)sm_count();
     count_launch();

@@ -220,10 +220,10 @@ __device__ __forceinline__ void load_tw(uint64_t* tw, const uint64_t* __restrict
     }
 }
 
+// Lets a launch of fn (a kernel without static shared memory) take `bytes` of
+// dynamic shared memory.
 inline cudaError_t set_smem(const void* fn, size_t bytes) {
-    if (bytes > 48 * 1024)
-        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return cudaSuccess;
+    return bytes > 48 * 1024 ? raise_smem_limit(fn) : cudaSuccess;
 }
 
 // Calls F.template operator()<L>() for the runtime L in [1, 12].
