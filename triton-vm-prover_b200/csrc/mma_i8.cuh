@@ -13,6 +13,7 @@
 // end, frees its TMEM and returns.
 #pragma once
 #include <cstdint>
+#include "bounded_wait.h"
 #include "field.cuh"
 
 namespace tvmc {
@@ -105,13 +106,7 @@ __device__ __forceinline__ bool mma8_try_wait(uint32_t bar, uint32_t parity) {
 // Waits for the group's MMAs (whole warps together); a wait that runs out sets dead.
 __device__ __forceinline__ void mma8_wait(uint32_t bar, uint32_t& phase, bool& dead) {
     if (!dead) {
-        bool done = mma8_try_wait(bar, phase);
-        if (!done) {
-            const long long t0 = clock64();
-            do done = mma8_try_wait(bar, phase);
-            while (!done && clock64() - t0 < MMA8_WAIT_CYCLES);
-        }
-        if (!done) {
+        if (!bounded_wait([&] { return mma8_try_wait(bar, phase); }, [] { return clock64(); }, MMA8_WAIT_CYCLES)) {
             atomicAdd(&g_mma8_timeouts, 1u);
             dead = true;
         }
