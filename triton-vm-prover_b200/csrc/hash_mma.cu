@@ -23,7 +23,7 @@ __device__ __forceinline__ uint32_t dyn_base() { return (uint32_t)__cvta_generic
 // Marks a commitment whose kernels timed out: word 0 of the heap tree's unused
 // node 0 (zero otherwise).
 __device__ __forceinline__ void mark_dead(const T5Mma& c, uint64_t* heap) {
-    if (c.dead && heap) heap[0] = 1;
+    if (c.waits.dead && heap) heap[0] = 1;
 }
 
 // Absorbs `perms` chunks of the row at p (element i at p[i * cs]): its n

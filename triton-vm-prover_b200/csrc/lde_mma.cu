@@ -73,9 +73,9 @@ struct Lm {
     uint8_t* a;      // the group's A tile
     uint32_t base;   // shared address of the map
     uint32_t tmem;   // this thread's D columns in its warp's lanes
-    uint32_t bar, phase;
+    uint32_t bar;
+    GroupWaits waits;
     int group, row, part;
-    bool dead;
 };
 
 // Byte offset of word j of line r in an A tile.
@@ -143,13 +143,13 @@ __device__ __forceinline__ void lm_init(Lm& c, const uint64_t* tw12) {
     c.a = c.sm + C::O_A + C::A_BYTES * c.group;
     c.bar = c.base + C::O_BAR + 8 * c.group;
     c.tmem = lds32(c.base + C::O_BAR + 32) + C::COLS * c.group + 64 * c.part + ((uint32_t)(c.row & ~31) << 16);
-    c.phase = 0;
-    c.dead = false;
+    c.waits = GroupWaits{};
 }
 
 // Every thread of the CTA calls this last.
 template <int B>
 __device__ __forceinline__ void lm_done(const Lm& c) {
+    if ((threadIdx.x & (LmCfg<B>::GROUP - 1)) == 0) mma8_drain(c.bar, c.waits);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -165,7 +165,7 @@ template <int B, class F>
 __device__ __forceinline__ void lm_dft(Lm& c, F&& out) {
     using C = LmCfg<B>;
     mma8_ready(c.group + 1, C::GROUP);
-    if ((threadIdx.x & (C::GROUP - 1)) == 0 && !c.dead) {
+    if ((threadIdx.x & (C::GROUP - 1)) == 0 && !c.waits.dead) {
         mma8_after();
         const uint64_t da = mma8_desc_sw128(c.base + C::O_A + C::A_BYTES * c.group), db = mma8_desc_sw128(c.base + C::O_B);
 #pragma unroll
@@ -174,7 +174,7 @@ __device__ __forceinline__ void lm_dft(Lm& c, F&& out) {
                                db + (k >> 2) * (C::B_HALF >> 4) + 2 * (k & 3), k > 0);
         mma8_commit(c.bar);
     }
-    mma8_wait(c.bar, c.phase, c.dead);
+    mma8_wait(c.bar, c.waits);
     uint32_t d[2][16];
     mma8_ld16(d[0], c.tmem);
 #pragma unroll

@@ -10,7 +10,8 @@
 //
 // Waits are bounded: after MMA8_WAIT_CYCLES a thread counts a timeout
 // (g_mma8_timeouts) and its group stops issuing; the kernel then runs to its
-// end, frees its TMEM and returns.
+// end, waits once more (bounded too) for the MMA it gave up on, frees its TMEM and
+// returns.
 #pragma once
 #include <cstdint>
 #include "bounded_wait.h"
@@ -103,17 +104,18 @@ __device__ __forceinline__ bool mma8_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return done != 0;
 }
-// Waits for the group's MMAs (whole warps together); a wait that runs out sets dead.
-__device__ __forceinline__ void mma8_wait(uint32_t bar, uint32_t& phase, bool& dead) {
-    if (!dead) {
-        if (!bounded_wait([&] { return mma8_try_wait(bar, phase); }, [] { return clock64(); }, MMA8_WAIT_CYCLES)) {
-            atomicAdd(&g_mma8_timeouts, 1u);
-            dead = true;
-        }
-    }
+// Waits for the group's MMAs (whole warps together).
+__device__ __forceinline__ void mma8_wait(uint32_t bar, GroupWaits& w) {
+    if (!group_wait(w, [&](uint32_t parity) { return mma8_try_wait(bar, parity); }, [] { return clock64(); },
+                    MMA8_WAIT_CYCLES))
+        atomicAdd(&g_mma8_timeouts, 1u);
     __syncwarp();
-    phase ^= 1;
     mma8_after();
+}
+// The group's issuing thread, before the barrier that precedes mma8_free.
+__device__ __forceinline__ void mma8_drain(uint32_t bar, const GroupWaits& w) {
+    group_drain(w, [&](uint32_t parity) { return mma8_try_wait(bar, parity); }, [] { return clock64(); },
+                MMA8_WAIT_CYCLES);
 }
 
 // 32 consecutive D columns of this thread's TMEM lane, complete on return (the

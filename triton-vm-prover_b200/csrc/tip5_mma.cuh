@@ -106,11 +106,10 @@ struct T5Mma {
     uint32_t a[T5M_WORDS / 2];  // shared addresses of this thread's word pairs in its A row
     uint32_t sbox;     // T5M_SBOX + lane * 4
     uint32_t tmem;     // this warp's lanes of the group's D columns
-    uint32_t phase;    // mbarrier parity of the next wait
+    GroupWaits waits;
     int group;
     int row;           // this thread's state within the group
     int part;          // and its part of it
-    bool dead;         // a wait of this thread ran out
 };
 
 // Value of the S-box table for a 32-bit word, byte by byte: the permute puts
@@ -204,12 +203,12 @@ __device__ __forceinline__ void t5m_init(T5Mma& c, uint32_t dyn) {
     c.sbox = T5M_SBOX + (tid & 31) * 4;
     asm volatile("" : "+r"(c.sbox)::"memory");  // no lookup moves above the barrier
     c.tmem = tb + 128 * c.group + 8 * T5M_WORDS * c.part + ((uint32_t)(c.row & ~31) << 16);
-    c.phase = 0;
-    c.dead = false;
+    c.waits = GroupWaits{};
 }
 
 // Every thread of the CTA calls this last.
 __device__ __forceinline__ void t5m_done(const T5Mma& c) {
+    if ((threadIdx.x & (T5M_GROUP - 1)) == 0) mma8_drain(c.base + T5M_BAR + 8 * c.group, c.waits);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -225,7 +224,7 @@ __device__ __forceinline__ void t5m_mds(uint64_t (&s)[T5M_WORDS], int rnd, T5Mma
     for (int i = 0; i < T5M_WORDS; i += 2) sts128(c.a[i / 2], s[i], s[i + 1]);
     mma8_ready(c.group + 1, T5M_GROUP);
     const uint32_t bar = c.base + T5M_BAR + 8 * c.group;
-    if ((threadIdx.x & (T5M_GROUP - 1)) == 0 && !c.dead) {
+    if ((threadIdx.x & (T5M_GROUP - 1)) == 0 && !c.waits.dead) {
         mma8_after();
         const uint32_t d = c.tmem;
         mma8_step<128>(d, mma8_desc_plain(c.base + T5M_ONES), mma8_desc_plain(c.base + T5M_RC + 4096 * rnd), 0);
@@ -234,7 +233,7 @@ __device__ __forceinline__ void t5m_mds(uint64_t (&s)[T5M_WORDS], int rnd, T5Mma
         for (int k = 0; k < 4; k++) mma8_step<128>(d, da + 2 * k, db + 2 * k, 1);
         mma8_commit(bar);
     }
-    mma8_wait(bar, c.phase, c.dead);
+    mma8_wait(bar, c.waits);
 #pragma unroll
     for (int h = 0; h < T5M_WORDS; h += 4) {
         uint32_t d[32];
