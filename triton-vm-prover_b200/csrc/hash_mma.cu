@@ -2,10 +2,10 @@
 // (tip5_mma.cuh).
 //
 // Two threads per sponge state; a group of 256 threads takes tiles of 128 rows,
-// four groups (one CTA of 1024 threads) fill an SM, and the grid is one CTA per
-// SM: tile i goes to group (i / gridDim) mod 4 of CTA i mod gridDim, so that a
-// last, partial wave is spread over all SMs.  Rows are read column-major (a warp
-// reads 32 consecutive rows of one column, 256 contiguous bytes).  Semantics:
+// and four groups (one CTA of 1024 threads) fill an SM.  A CTA ends after a bounded
+// number of tiles (TileSpan), so that kernels of other streams get in.  Rows are
+// read column-major (a warp reads 32 consecutive rows of one column, 256
+// contiguous bytes).  Semantics:
 // Tip5::hash_varlen (src/hash/tip5.cpp:246-282) -- zero state, overwrite the
 // rate with each full chunk and permute, last chunk = rest, 1, zeros.
 #include "hash_mma.h"
@@ -78,11 +78,40 @@ __device__ __forceinline__ void pair_hash(uint64_t (&s)[T5M_WORDS], const uint64
     t5m_permutation(s, c);
 }
 
-// The tiles of this thread's group.
+// How a launch's tiles go to its CTAs.  The CTAs form rounds of `ctas` (one per
+// SM); a round takes ctas * T5M_GROUPS * depth tiles, tile i of it by group
+// (i / ctas) mod T5M_GROUPS of CTA i mod ctas, so that a last, partial round is
+// spread over all SMs.
+struct TileSpan {
+    uint32_t tiles, ctas, depth;
+};
+// Permutations of a group before its CTA ends, 21 us each with all four groups at
+// work.  A CTA holds its SM's registers and shared memory until then, and only then
+// is a kernel of a greater-priority stream (an opening, a small request) dispatched
+// there.  Against the commit of 2^20 x 379 (x4), an opening took at most 43 ms with
+// one CTA per SM for the whole launch, 1.6 ms with 76 permutations and 1.0 with 38
+// (a commit of 2^10 x 379: 44, 4.9 and 2.7 ms); the row hash of 262144 x 379 took
+// 2.85, 2.91 and 2.92 ms in one build of each (a CTA's table fill is 8 us).
+constexpr uint32_t CTA_PERMS = 38;
+TileSpan tile_span(uint64_t tiles, uint64_t perms_per_tile, int sms) {
+    const uint32_t depth = (uint32_t)(CTA_PERMS / perms_per_tile);
+    return TileSpan{(uint32_t)tiles, (uint32_t)(tiles < (uint64_t)sms ? tiles : (uint64_t)sms), depth ? depth : 1};
+}
+uint32_t span_ctas(const TileSpan& s) {
+    const uint64_t round = (uint64_t)s.ctas * T5M_GROUPS * s.depth, rest = s.tiles % round;
+    return (uint32_t)(s.tiles / round * s.ctas + (rest < s.ctas ? rest : s.ctas));
+}
+
+// The tiles of this thread's group.  Each is formed anew from the block index: kept
+// across the permutations, the loop's bounds cost registers and 2% of the row hash.
 template <class F>
-__device__ __forceinline__ void for_tiles(const T5Mma& c, uint64_t tiles, F&& body) {
-    for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x * c.group; t < tiles; t += (uint64_t)gridDim.x * T5M_GROUPS)
-        body(t);
+__device__ __forceinline__ void for_tiles(const T5Mma& c, const TileSpan& s, F&& body) {
+    for (uint32_t k = 0; k < s.depth; k++) {
+        const uint32_t t = (blockIdx.x / s.ctas * s.depth + k) * (s.ctas * T5M_GROUPS) + blockIdx.x % s.ctas +
+                           s.ctas * c.group;
+        if (t >= s.tiles) break;
+        body((uint64_t)t);
+    }
 }
 
 }  // namespace
@@ -92,10 +121,11 @@ __device__ __forceinline__ void for_tiles(const T5Mma& c, uint64_t tiles, F&& bo
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_mma(const uint64_t* __restrict__ tab, uint64_t rstride,
                                                                   uint64_t cstride, uint64_t rows, uint32_t width,
                                                                   uint64_t* __restrict__ digests,
-                                                                  uint64_t* __restrict__ tree, int layout) {
+                                                                  uint64_t* __restrict__ tree, int layout,
+                                                                  TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
-    for_tiles(c, (rows + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+    for_tiles(c, span, [&](uint64_t tile) {
         const uint64_t row = tile * T5M_STATES + c.row;
         const bool live = row < rows;
         uint64_t s[T5M_WORDS];
@@ -110,10 +140,10 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_mma(const uint64_t
 // The same for up to HASH_MULTI_MAX tables: tile i belongs to the job j with
 // block0[j] <= i < block0[j + 1].
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_multi_mma(const __grid_constant__ HashJobs jobs,
-                                                                        uint32_t tiles) {
+                                                                        TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
-    for_tiles(c, tiles, [&](uint64_t tile) {
+    for_tiles(c, span, [&](uint64_t tile) {
         int j = 0;
         for (int k = 1; k < jobs.count; k++)
             if (jobs.j[k].block0 <= tile) j = k;
@@ -140,10 +170,10 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_multi_mma(const __
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_absorb_stripe_mma(const uint64_t* __restrict__ stripe, uint64_t L,
                                                                       uint32_t ncols, uint64_t* __restrict__ cap,
                                                                       int first, int last,
-                                                                      uint64_t* __restrict__ tree) {
+                                                                      uint64_t* __restrict__ tree, TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
-    for_tiles(c, (L + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+    for_tiles(c, span, [&](uint64_t tile) {
         const uint64_t row = tile * T5M_STATES + c.row;
         const bool live = row < L;
         uint64_t s[T5M_WORDS];
@@ -170,11 +200,11 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_absorb_stripe_mma(const uint
 
 // One tree level: parent p in [m/2, m) = hash_pair(node 2p, node 2p + 1).
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_level_mma(uint64_t* __restrict__ tree, uint64_t n,
-                                                                     uint64_t m, int layout) {
+                                                                     uint64_t m, int layout, TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
     const uint64_t parents = m >> 1;
-    for_tiles(c, (parents + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+    for_tiles(c, span, [&](uint64_t tile) {
         const uint64_t i = tile * T5M_STATES + c.row;
         const bool live = i < parents;
         const uint64_t par = parents + (live ? i : 0);
@@ -188,10 +218,11 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_level_mma(uint64_t* _
 
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_pairs_mma(const uint64_t* __restrict__ left,
                                                                    const uint64_t* __restrict__ right,
-                                                                   uint64_t* __restrict__ out, uint64_t count) {
+                                                                   uint64_t* __restrict__ out, uint64_t count,
+                                                                   TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
-    for_tiles(c, (count + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+    for_tiles(c, span, [&](uint64_t tile) {
         const uint64_t i = tile * T5M_STATES + c.row, k = i < count ? i : 0;
         uint64_t s[T5M_WORDS];
         pair_hash(s, left + 5 * k, right + 5 * k, c);
@@ -200,10 +231,11 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_pairs_mma(const uint64_
     t5m_done(c);
 }
 
-__global__ void __launch_bounds__(T5M_THREADS, 1) k_tip5_perm_mma(uint64_t* __restrict__ states, uint64_t count) {
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_tip5_perm_mma(uint64_t* __restrict__ states, uint64_t count,
+                                                                  TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
-    for_tiles(c, (count + T5M_STATES - 1) / T5M_STATES, [&](uint64_t tile) {
+    for_tiles(c, span, [&](uint64_t tile) {
         const uint64_t i = tile * T5M_STATES + c.row;
         const bool live = i < count;
         uint64_t s[T5M_WORDS];
@@ -221,16 +253,17 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_tip5_perm_mma(uint64_t* __re
 
 namespace {
 
-// One CTA per SM of the current device at most, no more than there are tiles.
+// kern(args..., span) over tiles of perms permutations each.
 template <class... P, class... A>
-cudaError_t launch(void (*kern)(P...), uint64_t tiles, cudaStream_t st, A... args) {
+cudaError_t launch(void (*kern)(P...), uint64_t tiles, uint64_t perms, cudaStream_t st, A... args) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)kern);
     if (e != cudaSuccess) return e;
+    const TileSpan span = tile_span(tiles, perms, sms);
     count_launch();
-    kern<<<(unsigned)(tiles < (uint64_t)sms ? tiles : (uint64_t)sms), T5M_THREADS, T5M_BYTES, st>>>(args...);
+    kern<<<span_ctas(span), T5M_THREADS, T5M_BYTES, st>>>(args..., span);
     return cudaGetLastError();
 }
 
@@ -240,29 +273,31 @@ uint64_t mma_tiles(uint64_t rows) { return (rows + T5M_STATES - 1) / T5M_STATES;
 
 cudaError_t launch_hash_rows_mma(const uint64_t* table, uint64_t rstride, uint64_t cstride, uint64_t rows,
                                  uint32_t width, uint64_t* digests, uint64_t* tree, int layout, cudaStream_t st) {
-    return launch(k_hash_rows_mma, mma_tiles(rows), st, table, rstride, cstride, rows, width, digests, tree, layout);
+    return launch(k_hash_rows_mma, mma_tiles(rows), width / T5_RATE + 1, st, table, rstride, cstride, rows, width, digests, tree, layout);
 }
 
 cudaError_t launch_hash_jobs_mma(const HashJobs& jobs, uint32_t tiles, cudaStream_t st) {
-    return launch(k_hash_rows_multi_mma, tiles, st, jobs, tiles);
+    uint32_t width = 0;
+    for (int k = 0; k < jobs.count; k++) width = jobs.j[k].width > width ? jobs.j[k].width : width;
+    return launch(k_hash_rows_multi_mma, tiles, width / T5_RATE + 1, st, jobs);
 }
 
 cudaError_t launch_absorb_stripe_mma(const uint64_t* stripe, uint64_t L, uint32_t ncols, uint64_t* cap, int first,
                                      int last, uint64_t* tree, cudaStream_t st) {
-    return launch(k_absorb_stripe_mma, mma_tiles(L), st, stripe, L, ncols, cap, first, last, tree);
+    return launch(k_absorb_stripe_mma, mma_tiles(L), ncols / T5_RATE + 1, st, stripe, L, ncols, cap, first, last, tree);
 }
 
 cudaError_t launch_merkle_level_mma(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st) {
-    return launch(k_merkle_level_mma, mma_tiles(m >> 1), st, tree, n, m, layout);
+    return launch(k_merkle_level_mma, mma_tiles(m >> 1), 1, st, tree, n, m, layout);
 }
 
 cudaError_t launch_hash_pairs_mma(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
                                   cudaStream_t st) {
-    return launch(k_hash_pairs_mma, mma_tiles(count), st, left, right, out, count);
+    return launch(k_hash_pairs_mma, mma_tiles(count), 1, st, left, right, out, count);
 }
 
 cudaError_t launch_tip5_permutations_mma(uint64_t* states, uint64_t count, cudaStream_t st) {
-    return launch(k_tip5_perm_mma, mma_tiles(count), st, states, count);
+    return launch(k_tip5_perm_mma, mma_tiles(count), 1, st, states, count);
 }
 
 unsigned int mma_timeouts() {
