@@ -78,3 +78,35 @@ def test_multi_commit_rejects_bad_tables(tv):
     with pytest.raises(tv.InvalidArgument):
         tv.commit_multi([good], expansion=3)
     assert tv.commit_multi([]) == []
+
+
+@pytest.mark.parametrize("heights", [[256] * 63 + [2], [256] * 64, [1 << 14] + [1] * 5 + [2, 4, 128, 64],
+                                     [1 << 13, 1 << 13, 64]])
+def test_multi_commit_trees_at_the_edge_of_the_rule(tv, oracle, heights):
+    """Parents of all trees together just below and at the tensor-core form's least,
+    with trees of a single row, and of less than one tile or chunk, among them."""
+    traces = [rand_u64(8600 + i, (1, h)) for i, h in enumerate(heights)]
+    cs = tv.commit_multi(traces, expansion=1)
+    try:
+        for t, c in zip(traces, cs):
+            exp = oracle.merkle(oracle.hash_rows_cm(oracle.lde(t, 1, 7)))
+            assert (c.nodes()[1:] == exp[1:]).all()
+    finally:
+        for c in cs:
+            c.free()
+
+
+def test_multi_commit_trees_share_their_launches(tv):
+    """The launches above the leaves do not grow with the number of tables."""
+    def launches(count):
+        traces = [to_dev(rand_u64(8700 + i, (3, 1 << 11))) for i in range(count)]
+        before = tv.lib().tvmc_launch_count()
+        cs = tv.commit_multi([t.data_ptr() for t in traces], device_ptr=True, shapes=[(1 << 11, 3)] * count, sync=True)
+        after = tv.lib().tvmc_launch_count()
+        for c in cs:
+            c.free()
+        return after - before - count  # one LDE launch each
+
+    assert launches(1) == 3   # rows, two launches of seven levels
+    assert launches(16) <= 8  # rows, four wide levels of all trees, two launches above
+    assert launches(64) <= 10

@@ -117,21 +117,20 @@ __global__ void __launch_bounds__(COOP_TREE_THREADS) k_merkle_coop(uint64_t* __r
     subtree(tree, n, m, layout, levels, blockIdx.x, sd, c);
 }
 
-// The tops of several heap trees, one CTA per tree: tree j has its level of
-// m[j] <= MULTI_TOP_MAX_NODES nodes in place and gets every level above it,
-// COOP_TREE_LEVELS of them at a time.
-__global__ void __launch_bounds__(COOP_TREE_THREADS) k_merkle_tops_coop(const __grid_constant__ TopJobs jobs) {
+// Several heap trees; CTA b belongs to job j with block0[j] <= b < block0[j + 1].
+__global__ void __launch_bounds__(COOP_TREE_THREADS) k_merkle_levels_coop(const __grid_constant__ LevelJobs jobs) {
     __shared__ T5CoopTables tables;
     __shared__ double2 xch[COOP_TREE_STATES * 2 * T5_STATE];
     __shared__ uint64_t sd[5 * (COOP_TREE_NODES + COOP_TREE_NODES / 2)];
     T5Coop c;
     t5c_init(c, tables, xch);
-    uint64_t* tree = jobs.j[blockIdx.x].tree;
-    for (uint64_t m = jobs.j[blockIdx.x].m; m > 1;) {
-        const int lg = 63 - __clzll((long long)m), levels = lg < COOP_TREE_LEVELS ? lg : COOP_TREE_LEVELS;
-        for (uint64_t k = 0; k * COOP_TREE_NODES < m; k++) subtree(tree, m, m, LAYOUT_HEAP, levels, k, sd, c);
-        m >>= levels;
-    }
+    int j = 0;
+    for (int k = 1; k < jobs.count; k++)
+        if (jobs.j[k].block0 <= blockIdx.x) j = k;
+    const uint64_t m = jobs.j[j].m;
+    const int lg = 63 - __clzll((long long)m);
+    subtree(jobs.j[j].tree, m, m, LAYOUT_HEAP, lg < COOP_TREE_LEVELS ? lg : COOP_TREE_LEVELS,
+            blockIdx.x - jobs.j[j].block0, sd, c);
 }
 
 __global__ void __launch_bounds__(COOP_THREADS) k_hash_pairs_coop(const uint64_t* __restrict__ left,
@@ -233,14 +232,13 @@ uint64_t coop_blocks(uint64_t rows) { return blocks_of(rows); }
 
 cudaError_t launch_merkle_coop(uint64_t* tree, uint64_t n, uint64_t m, int layout, int levels, cudaStream_t st) {
     count_launch();
-    k_merkle_coop<<<(unsigned)((m + COOP_TREE_NODES - 1) / COOP_TREE_NODES), COOP_TREE_THREADS, 0, st>>>(tree, n, m,
-                                                                                                     layout, levels);
+    k_merkle_coop<<<(unsigned)coop_tree_blocks(m), COOP_TREE_THREADS, 0, st>>>(tree, n, m, layout, levels);
     return cudaGetLastError();
 }
 
-cudaError_t launch_merkle_tops_coop(const TopJobs& jobs, int count, cudaStream_t st) {
+cudaError_t launch_merkle_levels_coop(const LevelJobs& jobs, uint32_t blocks, cudaStream_t st) {
     count_launch();
-    k_merkle_tops_coop<<<(unsigned)count, COOP_TREE_THREADS, 0, st>>>(jobs);
+    k_merkle_levels_coop<<<blocks, COOP_TREE_THREADS, 0, st>>>(jobs);
     return cudaGetLastError();
 }
 

@@ -216,6 +216,27 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_level_mma(uint64_t* _
     t5m_done(c);
 }
 
+// The same for up to HASH_MULTI_MAX heap trees; tiles as in k_hash_rows_multi_mma.
+__global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_levels_mma(const __grid_constant__ LevelJobs jobs,
+                                                                      TileSpan span) {
+    T5Mma c;
+    t5m_init(c, dyn_base());
+    for_tiles(c, span, [&](uint64_t tile) {
+        int j = 0;
+        for (int k = 1; k < jobs.count; k++)
+            if (jobs.j[k].block0 <= tile) j = k;
+        uint64_t* tree = jobs.j[j].tree;
+        const uint64_t parents = jobs.j[j].m >> 1, i = (tile - jobs.j[j].block0) * T5M_STATES + c.row;
+        const bool live = i < parents;
+        const uint64_t par = parents + (live ? i : 0);
+        uint64_t s[T5M_WORDS];
+        pair_hash(s, tree + 10 * par, tree + 10 * par + 5, c);
+        if (live) store_digest(s, tree + 5 * par, c);
+        mark_dead(c, tree);
+    });
+    t5m_done(c);
+}
+
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_pairs_mma(const uint64_t* __restrict__ left,
                                                                    const uint64_t* __restrict__ right,
                                                                    uint64_t* __restrict__ out, uint64_t count,
@@ -289,6 +310,10 @@ cudaError_t launch_absorb_stripe_mma(const uint64_t* stripe, uint64_t L, uint32_
 
 cudaError_t launch_merkle_level_mma(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st) {
     return launch(k_merkle_level_mma, mma_tiles(m >> 1), 1, st, tree, n, m, layout);
+}
+
+cudaError_t launch_merkle_levels_mma(const LevelJobs& jobs, uint32_t tiles, cudaStream_t st) {
+    return launch(k_merkle_levels_mma, tiles, 1, st, jobs);
 }
 
 cudaError_t launch_hash_pairs_mma(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,

@@ -14,6 +14,8 @@ cudaError_t launch_absorb_stripe_mma(const uint64_t* stripe, uint64_t L, uint32_
                                      int last, uint64_t* tree, cudaStream_t st);
 // The level of m/2 parents above the m nodes [m, 2m) in place.
 cudaError_t launch_merkle_level_mma(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st);
+// The same for several heap trees; block0 counts tiles of 128 parents, `tiles` in all.
+cudaError_t launch_merkle_levels_mma(const LevelJobs& jobs, uint32_t tiles, cudaStream_t st);
 uint64_t mma_tiles(uint64_t rows);
 cudaError_t launch_hash_pairs_mma(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
                                   cudaStream_t st);

@@ -92,8 +92,8 @@ cudaError_t launch_absorb_stripe(const uint64_t* stripe, uint64_t L, uint32_t nc
 cudaError_t launch_hash_pairs(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
                               cudaStream_t st);
 
-// Multi-table row hash + heap Merkle trees (one launch for up to
-// HASH_MULTI_MAX tables, one more for the small tree tops).
+// Multi-table row hash + heap Merkle trees: every launch takes all of up to
+// HASH_MULTI_MAX tables, the rows first and then the trees' levels.
 struct MultiHashTable {
     const uint64_t* lde;  // column-major, column stride L
     uint64_t* tree;       // heap layout, 2L digests (node 0 unused)
@@ -101,7 +101,6 @@ struct MultiHashTable {
     uint32_t width;
 };
 constexpr int HASH_MULTI_MAX = 64;
-constexpr uint64_t MULTI_TOP_MAX_NODES = 1024;  // larger tree tops use the single-tree kernels
 struct HashJob {
     const uint64_t* lde;
     uint64_t* tree;
@@ -113,12 +112,14 @@ struct HashJobs {
     HashJob j[HASH_MULTI_MAX];
     int count;
 };
-struct TopJob {
+struct LevelJob {  // one heap tree of a launch that builds levels of several
     uint64_t* tree;
-    uint64_t m;  // nodes of the level already in place
+    uint64_t m;       // the nodes [m, 2m) are in place, m > 1
+    uint32_t block0;  // first tile or CTA of this tree
 };
-struct TopJobs {
-    TopJob j[HASH_MULTI_MAX];
+struct LevelJobs {
+    LevelJob j[HASH_MULTI_MAX];
+    int count;
 };
 cudaError_t launch_hash_rows_multi(const MultiHashTable* tabs, int count, cudaStream_t st);
 cudaError_t launch_tip5_permutations(uint64_t* states, uint64_t count, cudaStream_t st);
