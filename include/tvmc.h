@@ -23,6 +23,13 @@
  *     most recent failure on the calling thread.
  *   - Thread safety: the library is safe to call from several threads; one
  *     commitment handle must not be used from two threads at once.
+ *   - Device waits are bounded (about a second; only a failing GPU exceeds it).
+ *     When one runs out the kernel goes on and its results are not valid: the
+ *     calls that return host data, and every call that waits for a commitment
+ *     or reads from it, then return TVMC_ERR_TIMEOUT.  The *_gpu calls, the
+ *     device pointers of a commitment and tvmc_commitment_absorb_root are
+ *     enqueued before the kernels end and cannot: a caller of those looks at
+ *     tvmc_get_tuning("mma_timeouts"), or syncs the commitment.
  *   - The first call on a device builds twiddle tables with synchronous copies;
  *     make one call before capturing work into a CUDA graph.
  *
@@ -226,6 +233,9 @@ typedef struct tvmc_commitment tvmc_commitment;
  *   "fail_alloc_after"    fault injection for tests: k > 0 makes the k-th device allocation the
  *                         library requests from now on fail as out-of-memory (once, on the host,
  *                         without reaching the driver); 0 disables
+ *   "fail_mma_after"      the same for device waits: the k-th launch of a tensor-core kernel from
+ *                         now on (a captured one every time it runs) reports a wait that ran out,
+ *                         though none did; 0 disables
  * Unknown keys return TVMC_ERR_INVALID.  tvmc_get_tuning also reads "pool_used_bytes": the bytes
  * currently allocated from the current device's stream-ordered pool (a leak check), and
  * "mma_timeouts": tensor-core waits that gave up (after about a second; 0 unless a GPU fails). */
@@ -311,8 +321,7 @@ int tvmc_sponge_absorb_gpu(uint64_t* d_state, const uint64_t* d_data, size_t len
  * (discriminant 0, then the 5 root words), into d_state on `stream`, ordered
  * after the commitment: the root never visits the host (src/gpu/gpu_stark.cu:2577-2585). */
 int tvmc_commitment_absorb_root(tvmc_commitment* c, uint64_t* d_state, void* stream);
-/* Wait for the commitment and copy its root (5 words) to host memory; TVMC_ERR_TIMEOUT if one of its
- * hash kernels gave up waiting. */
+/* Wait for the commitment and copy its root (5 words) to host memory. */
 int tvmc_commitment_root(tvmc_commitment* c, uint64_t* root);
 int tvmc_commitment_sync(tvmc_commitment* c);
 /* Sizes: LDE length (= number of leaves) and width. */
@@ -420,8 +429,9 @@ int tvmc_server_submit_randomized(tvmc_server* s, const uint64_t* trace, size_t 
                                   const uint64_t* randomizers, size_t num_randomizers, uint32_t flags,
                                   uint64_t* request_id);
 /* Wait until the request is committed (timeout_ms < 0: no limit; expiry returns
- * TVMC_ERR_TIMEOUT) and copy its root; a request whose footprint exceeds the
- * whole budget fails with TVMC_ERR_NOMEM. */
+ * TVMC_ERR_TIMEOUT) and copy its root (root may be NULL); a request whose
+ * footprint exceeds the whole budget fails with TVMC_ERR_NOMEM, one of whose
+ * device waits ran out with TVMC_ERR_CUDA. */
 int tvmc_server_wait(tvmc_server* s, uint64_t request_id, int64_t timeout_ms, uint64_t* root);
 /* Openings of a committed request from its device-resident tree: auth paths
  * (count x height x 5 words, as tvmc_commitment_auth_paths) and, when the

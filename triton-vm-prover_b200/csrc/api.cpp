@@ -65,10 +65,16 @@ int cuda_fail(cudaError_t e, const char* where) {
 // the GPU itself sees nothing.
 std::atomic<long long> g_fail_alloc_after{0};
 
-bool injected_alloc_failure() {
-    long long k = g_fail_alloc_after.load();
+// Device-wait failure injection (tuning key "fail_mma_after" = k > 0): the status
+// word of the k-th tensor-core launch from then on is set behind the kernel, once,
+// as the kernel does when a wait runs out.  The kernel itself runs as ever.
+std::atomic<long long> g_fail_mma_after{0};
+
+// Counts k down to zero; true on the step from 1.
+bool count_down(std::atomic<long long>& left) {
+    long long k = left.load();
     while (k > 0) {
-        if (g_fail_alloc_after.compare_exchange_weak(k, k - 1)) return k == 1;
+        if (left.compare_exchange_weak(k, k - 1)) return k == 1;
     }
     return false;
 }
@@ -76,12 +82,12 @@ bool injected_alloc_failure() {
 // Every device allocation of this file goes through these two.
 template <class T>
 cudaError_t dev_malloc(T** p, size_t bytes) {
-    if (injected_alloc_failure()) return cudaErrorMemoryAllocation;
+    if (count_down(g_fail_alloc_after)) return cudaErrorMemoryAllocation;
     return cudaMalloc((void**)p, bytes);
 }
 template <class T>
 cudaError_t dev_malloc_async(T** p, size_t bytes, cudaStream_t st) {
-    if (injected_alloc_failure()) return cudaErrorMemoryAllocation;
+    if (count_down(g_fail_alloc_after)) return cudaErrorMemoryAllocation;
     return cudaMallocAsync((void**)p, bytes, st);
 }
 
@@ -216,6 +222,29 @@ int get_plan(int logn, int le, uint64_t offset, LdePlan* pl) {
         pl->sc_hi = T.sc[key].second;
     }
     return TVMC_OK;
+}
+
+constexpr const char* RAN_OUT = "a device wait ran out: the result is not valid";
+
+// The status word of calls that return host data: pinned, so that a kernel that
+// gives up writes it and the others cost nothing.  One per thread; a call clears
+// it, launches with it, and checks it once its kernels are done.
+struct HostStatus {
+    uint64_t* word = nullptr;
+    ~HostStatus() {
+        if (word) cudaFreeHost(word);
+    }
+};
+thread_local HostStatus t_status;
+
+int clear_status(uint64_t** word) {
+    if (!t_status.word) CK(cudaHostAlloc((void**)&t_status.word, 8, cudaHostAllocPortable | cudaHostAllocMapped));
+    *t_status.word = 0;
+    *word = t_status.word;
+    return TVMC_OK;
+}
+int check_status(const uint64_t* word) {
+    return *(const volatile uint64_t*)word ? fail(TVMC_ERR_TIMEOUT, RAN_OUT) : TVMC_OK;
 }
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -353,7 +382,7 @@ void give_slot_event(cudaStream_t st, int kind, cudaEvent_t ev) {
 }
 
 int run_lde(const LdePlan& pl, const uint64_t* d_tr, uint64_t tld, uint64_t* d_out, uint64_t old, size_t width,
-            cudaStream_t st, const RandAdd& ra = RandAdd{}) {
+            cudaStream_t st, uint64_t* status, const RandAdd& ra = RandAdd{}) {
     size_t chunk = lde_chunk_cols(pl.logn, pl.log_exp, width);
     uint64_t* scratch = nullptr;
     int rc = stream_scratch(st, lde_scratch_words(pl.logn, pl.log_exp, chunk), &scratch);
@@ -361,7 +390,7 @@ int run_lde(const LdePlan& pl, const uint64_t* d_tr, uint64_t tld, uint64_t* d_o
     for (size_t c0 = 0; c0 < width; c0 += chunk) {
         size_t nc = std::min(chunk, width - c0);
         cudaError_t e =
-            launch_lde(pl, d_tr + c0 * tld, tld, d_out + c0 * old, old, nc, scratch, st, ra.cols(c0), ra.rm);
+            launch_lde(pl, d_tr + c0 * tld, tld, d_out + c0 * old, old, nc, scratch, st, status, ra.cols(c0), ra.rm);
         if (e != cudaSuccess) return cuda_fail(e, "launch_lde");
     }
     return TVMC_OK;
@@ -398,7 +427,7 @@ int copy_stream(cudaStream_t compute, cudaStream_t* out) {
 constexpr int UPLOAD_STAGES = 4;
 constexpr int stage_kind(int b) { return b < 2 ? 1 + b : 16 + b; }
 int upload_lde_pipelined(const LdePlan& pl, const uint64_t* h_trace, size_t n, size_t width, uint64_t* d_out,
-                         size_t L, cudaStream_t st, const RandAdd& ra = RandAdd{}) {
+                         size_t L, cudaStream_t st, uint64_t* status, const RandAdd& ra = RandAdd{}) {
     cudaStream_t cs = nullptr;
     int rc = copy_stream(st, &cs);
     if (rc) return rc;
@@ -434,7 +463,8 @@ int upload_lde_pipelined(const LdePlan& pl, const uint64_t* h_trace, size_t n, s
             e = cudaMemcpyAsync(stage[b], h_trace + c0 * n, nc * n * 8, cudaMemcpyHostToDevice, cs);
         if (e == cudaSuccess) e = cudaEventRecord(ready[b], cs);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ready[b], 0);
-        if (e == cudaSuccess) e = launch_lde(pl, stage[b], n, d_out + c0 * L, L, nc, scratch, st, ra.cols(c0), ra.rm);
+        if (e == cudaSuccess)
+            e = launch_lde(pl, stage[b], n, d_out + c0 * L, L, nc, scratch, st, status, ra.cols(c0), ra.rm);
         if (e == cudaSuccess) e = cudaEventRecord(freed[b], st);
     }
     for (int b = 0; b < nst; b++) {
@@ -451,7 +481,7 @@ int upload_lde_pipelined(const LdePlan& pl, const uint64_t* h_trace, size_t n, s
     return TVMC_OK;
 }
 
-int ntt_impl(uint64_t* d, size_t n, size_t cols, int inverse, cudaStream_t st) {
+int ntt_impl(uint64_t* d, size_t n, size_t cols, int inverse, cudaStream_t st, uint64_t* status) {
     if (!is_pow2(n)) return fail(TVMC_ERR_INVALID, "NTT size must be a power of 2 (got %zu)", n);
     int l = log2u(n);
     if (l > MAX_LOG_NTT) return fail(TVMC_ERR_UNSUPPORTED, "NTT size 2^%d exceeds 2^%d", l, MAX_LOG_NTT);
@@ -461,7 +491,7 @@ int ntt_impl(uint64_t* d, size_t n, size_t cols, int inverse, cudaStream_t st) {
     if (rc) return rc;
     uint64_t* scratch = nullptr;
     if ((rc = stream_scratch(st, ntt_scratch_words(l, cols), &scratch))) return rc;
-    cudaError_t e = launch_ntt(pl, inverse, d, n, cols, scratch, st);
+    cudaError_t e = launch_ntt(pl, inverse, d, n, cols, scratch, st, status);
     if (e != cudaSuccess) return cuda_fail(e, "launch_ntt");
     return TVMC_OK;
 }
@@ -578,7 +608,7 @@ int commit_frugal(const LdePlan& pl, const uint64_t* trace, bool dev, bool rm, s
         const bool last = c0 + nc == width;
         for (size_t k = 0; k < nc && e == cudaSuccess; k += chunk) {
             const size_t kc = std::min(chunk, nc - k);
-            e = launch_lde(pl, src + (c0 + k) * n, n, stripe + k * L, L, kc, scratch, st, ra.cols(c0 + k), ra.rm);
+            e = launch_lde(pl, src + (c0 + k) * n, n, stripe + k * L, L, kc, scratch, st, nodes, ra.cols(c0 + k), ra.rm);
         }
         if (e == cudaSuccess) e = launch_absorb_stripe(stripe, L, (uint32_t)nc, cap, first, last, nodes, st);
         first = false;
@@ -626,6 +656,11 @@ int tvmc::check_lde_sizes(size_t trace_len, size_t extended_len, int* logn, int*
     return TVMC_OK;
 }
 
+cudaError_t tvmc::mma_launched(uint64_t* status, cudaStream_t st) {
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess && count_down(g_fail_mma_after) && status ? cudaMemsetAsync(status, 1, 1, st) : e;
+}
+
 int tvmc::set_error(int code, const char* msg) {
     g_err = msg;
     return code;
@@ -638,6 +673,9 @@ struct tvmc_commitment {
     uint64_t* d_lde = nullptr;
     uint64_t* d_nodes = nullptr;
     cudaEvent_t done = nullptr;
+    // the status word (node 0) was read as zero after `done`: no kernel of this
+    // commitment gave up.  tvmc_batch_run, which computes it anew, clears it.
+    std::atomic<bool> sound{false};
     // TVMC_PROFILE: events at start / after upload / after LDE / after hash+tree
     cudaEvent_t prof[4] = {nullptr, nullptr, nullptr, nullptr};
     bool batch_owned = false;  // freed by tvmc_batch_free only
@@ -707,15 +745,32 @@ struct tvmc_batch {
 };
 
 namespace {
+// Waits for the commitment: TVMC_ERR_TIMEOUT if one of its kernels gave up, in which
+// case nothing of it is handed out.  With `root` also its root, in the same copy.
+int wait_sound(tvmc_commitment* c, uint64_t* root = nullptr) {
+    if (c->sound.load() && !root) return TVMC_OK;
+    cudaStream_t st;
+    int rc = acc_stream(&st);
+    if (rc) return rc;
+    uint64_t head[10];  // node 0, the status word in front, and node 1
+    CK(cudaStreamWaitEvent(st, c->done, 0));
+    CK(cudaMemcpyAsync(head, c->d_nodes, sizeof head, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (head[0]) return fail(TVMC_ERR_TIMEOUT, RAN_OUT);
+    c->sound = true;
+    if (root) std::memcpy(root, head + 5, 40);
+    return TVMC_OK;
+}
+
 // Index list -> device, a gather kernel, result -> host, all on the calling
 // thread's accessor stream after the commitment's completion event; per_item
 // output words per index.
 template <typename Gather>
-int gather_sync(const tvmc_commitment* c, const void* idx, size_t count, size_t per_item, uint64_t* out,
-                Gather gather) {
+int gather_sync(tvmc_commitment* c, const void* idx, size_t count, size_t per_item, uint64_t* out, Gather gather) {
     static_assert(sizeof(size_t) == 8, "64-bit indices");
     cudaStream_t st;
-    int rc = acc_stream(&st);
+    int rc = wait_sound(c);
+    if (!rc) rc = acc_stream(&st);
     if (rc) return rc;
     HostBuf hb;
     if ((rc = host_buf(count * (1 + per_item), &hb))) return rc;
@@ -729,9 +784,10 @@ int gather_sync(const tvmc_commitment* c, const void* idx, size_t count, size_t 
 }
 
 // Device words -> host after the commitment's completion, on the accessor stream.
-int read_sync(const tvmc_commitment* c, const uint64_t* src, size_t words, uint64_t* out) {
+int read_sync(tvmc_commitment* c, const uint64_t* src, size_t words, uint64_t* out) {
     cudaStream_t st;
-    int rc = acc_stream(&st);
+    int rc = wait_sound(c);
+    if (!rc) rc = acc_stream(&st);
     if (rc) return rc;
     CK(cudaStreamWaitEvent(st, c->done, 0));
     CK(cudaMemcpyAsync(out, src, words * 8, cudaMemcpyDeviceToHost, st));
@@ -858,6 +914,7 @@ int tvmc_set_tuning(const char* key, long long value) {
         g_tune_tile_log = value;
     } else if (!strcmp(key, "hash_unfused_tree")) g_tune_unfused_tree = value ? 1 : 0;
     else if (!strcmp(key, "fail_alloc_after")) g_fail_alloc_after = value;
+    else if (!strcmp(key, "fail_mma_after")) g_fail_mma_after = value;
     else return fail(TVMC_ERR_INVALID, "unknown tuning key '%s'", key);
     return TVMC_OK;
 }
@@ -877,6 +934,7 @@ int tvmc_get_tuning(const char* key, long long* value) {
     else if (!strcmp(key, "mma_timeouts")) *value = (long long)mma_timeouts() + lde_mma_timeouts();
     else if (!strcmp(key, "ntt_tile_log")) *value = g_tune_tile_log;
     else if (!strcmp(key, "fail_alloc_after")) *value = g_fail_alloc_after;
+    else if (!strcmp(key, "fail_mma_after")) *value = g_fail_mma_after;
     else if (!strcmp(key, "pool_used_bytes")) {
         int dev;
         cudaMemPool_t pool;
@@ -901,10 +959,10 @@ int tvmc_device_count(void) {
 // ---------------------------------------------------------------- NTT
 
 int tvmc_ntt_forward_batched_gpu(uint64_t* d_data, size_t n, size_t num_cols, void* stream) {
-    return ntt_impl(d_data, n, num_cols, 0, as_stream(stream));
+    return ntt_impl(d_data, n, num_cols, 0, as_stream(stream), nullptr);
 }
 int tvmc_ntt_inverse_batched_gpu(uint64_t* d_data, size_t n, size_t num_cols, void* stream) {
-    return ntt_impl(d_data, n, num_cols, 1, as_stream(stream));
+    return ntt_impl(d_data, n, num_cols, 1, as_stream(stream), nullptr);
 }
 
 int tvmc_ntt_host(uint64_t* data, size_t n, size_t num_cols, int inverse) {
@@ -912,21 +970,27 @@ int tvmc_ntt_host(uint64_t* data, size_t n, size_t num_cols, int inverse) {
     DBuf d;
     CK(d.alloc(n * num_cols));
     CK(cudaMemcpy(d.p, data, n * num_cols * 8, cudaMemcpyHostToDevice));
-    int rc = ntt_impl(d.p, n, num_cols, inverse, nullptr);
+    uint64_t* status = nullptr;
+    int rc = clear_status(&status);
+    if (!rc) rc = ntt_impl(d.p, n, num_cols, inverse, nullptr, status);
     if (rc) return rc;
     CK(cudaMemcpy(data, d.p, n * num_cols * 8, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
-int tvmc_evaluate_on_coset_gpu(const uint64_t* d_coeffs, size_t num_coeffs, size_t num_cols, uint64_t* d_out,
-                               size_t domain_len, uint64_t offset, void* stream) {
+static int coset_impl(const uint64_t* d_coeffs, size_t num_coeffs, size_t num_cols, uint64_t* d_out,
+                      size_t domain_len, uint64_t offset, cudaStream_t st, uint64_t* status) {
     if (!is_pow2(domain_len)) return fail(TVMC_ERR_INVALID, "NTT size must be a power of 2 (got %zu)", domain_len);
     if (log2u(domain_len) > MAX_LOG_NTT)
         return fail(TVMC_ERR_UNSUPPORTED, "NTT size 2^%d exceeds 2^%d", log2u(domain_len), MAX_LOG_NTT);
     if (num_cols == 0) return TVMC_OK;
-    cudaStream_t st = as_stream(stream);
     CK(launch_coset_scale(d_coeffs, num_coeffs, num_coeffs, d_out, domain_len, num_cols, offset, st));
-    return ntt_impl(d_out, domain_len, num_cols, 0, st);
+    return ntt_impl(d_out, domain_len, num_cols, 0, st, status);
+}
+
+int tvmc_evaluate_on_coset_gpu(const uint64_t* d_coeffs, size_t num_coeffs, size_t num_cols, uint64_t* d_out,
+                               size_t domain_len, uint64_t offset, void* stream) {
+    return coset_impl(d_coeffs, num_coeffs, num_cols, d_out, domain_len, offset, as_stream(stream), nullptr);
 }
 
 int tvmc_evaluate_on_coset_host(const uint64_t* coeffs, size_t num_coeffs, size_t num_cols, uint64_t* out,
@@ -936,11 +1000,12 @@ int tvmc_evaluate_on_coset_host(const uint64_t* coeffs, size_t num_coeffs, size_
     HostBuf hb;
     int rc = host_buf(num_cols * (num_coeffs + domain_len), &hb);
     if (rc) return rc;
-    uint64_t *a = hb.p, *b = a + num_cols * num_coeffs;
+    uint64_t *a = hb.p, *b = a + num_cols * num_coeffs, *status = nullptr;
+    if ((rc = clear_status(&status))) return rc;
     if (num_coeffs) CK(cudaMemcpy(a, coeffs, 8 * num_cols * num_coeffs, cudaMemcpyHostToDevice));
-    if ((rc = tvmc_evaluate_on_coset_gpu(a, num_coeffs, num_cols, b, domain_len, offset, nullptr))) return rc;
+    if ((rc = coset_impl(a, num_coeffs, num_cols, b, domain_len, offset, nullptr, status))) return rc;
     CK(cudaMemcpy(out, b, 8 * num_cols * domain_len, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
 int tvmc_rowmajor_to_colmajor_gpu(const uint64_t* d_in, size_t rows, size_t cols, uint64_t* d_out, void* stream) {
@@ -952,16 +1017,22 @@ int tvmc_rowmajor_to_colmajor_gpu(const uint64_t* d_in, size_t rows, size_t cols
 
 // ---------------------------------------------------------------- LDE
 
-int tvmc_lde_batch_gpu(const uint64_t* d_traces, size_t num_columns, size_t trace_len, uint64_t* d_extended,
-                       size_t extended_len, uint64_t trace_offset, uint64_t extended_offset, void* stream) {
-    (void)trace_offset;
+static int lde_impl(const uint64_t* d_traces, size_t num_columns, size_t trace_len, uint64_t* d_extended,
+                    size_t extended_len, uint64_t extended_offset, cudaStream_t st, uint64_t* status) {
     int logn, le;
     int rc = check_lde_sizes(trace_len, extended_len, &logn, &le);
     if (rc) return rc;
     if (num_columns == 0) return TVMC_OK;
     LdePlan pl;
     if ((rc = get_plan(logn, le, extended_offset, &pl))) return rc;
-    return run_lde(pl, d_traces, trace_len, d_extended, extended_len, num_columns, as_stream(stream));
+    return run_lde(pl, d_traces, trace_len, d_extended, extended_len, num_columns, st, status);
+}
+
+int tvmc_lde_batch_gpu(const uint64_t* d_traces, size_t num_columns, size_t trace_len, uint64_t* d_extended,
+                       size_t extended_len, uint64_t trace_offset, uint64_t extended_offset, void* stream) {
+    (void)trace_offset;
+    return lde_impl(d_traces, num_columns, trace_len, d_extended, extended_len, extended_offset, as_stream(stream),
+                    nullptr);
 }
 
 int tvmc_lde_host(const uint64_t* traces, size_t num_columns, size_t trace_len, uint64_t* extended,
@@ -974,16 +1045,17 @@ int tvmc_lde_host(const uint64_t* traces, size_t num_columns, size_t trace_len, 
     CK(a.alloc(trace_len * num_columns));
     CK(b.alloc(extended_len * num_columns));
     CK(cudaMemcpy(a.p, traces, trace_len * num_columns * 8, cudaMemcpyHostToDevice));
-    if ((rc = tvmc_lde_batch_gpu(a.p, num_columns, trace_len, b.p, extended_len, 1, extended_offset, nullptr)))
-        return rc;
+    uint64_t* status = nullptr;
+    if ((rc = clear_status(&status))) return rc;
+    if ((rc = lde_impl(a.p, num_columns, trace_len, b.p, extended_len, extended_offset, nullptr, status))) return rc;
     CK(cudaMemcpy(extended, b.p, extended_len * num_columns * 8, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
-int tvmc_lde_randomized_gpu(const uint64_t* d_traces, size_t num_columns, size_t trace_len,
-                            const uint64_t* d_randomizers, size_t num_randomizers, uint64_t* d_extended,
-                            size_t extended_len, uint64_t trace_offset, uint64_t extended_offset, uint32_t flags,
-                            void* stream) {
+static int lde_randomized_impl(const uint64_t* d_traces, size_t num_columns, size_t trace_len,
+                               const uint64_t* d_randomizers, size_t num_randomizers, uint64_t* d_extended,
+                               size_t extended_len, uint64_t trace_offset, uint64_t extended_offset, uint32_t flags,
+                               cudaStream_t st, uint64_t* status) {
     int logn, le;
     int rc = check_lde_sizes(trace_len, extended_len, &logn, &le);
     if (rc) return rc;
@@ -991,7 +1063,6 @@ int tvmc_lde_randomized_gpu(const uint64_t* d_traces, size_t num_columns, size_t
     if (trace_offset % P == 0) return fail(TVMC_ERR_INVALID, "trace offset must be nonzero mod p");
     if (num_columns == 0) return TVMC_OK;
     if (num_randomizers && !d_randomizers) return fail(TVMC_ERR_INVALID, "null randomizers");
-    cudaStream_t st = as_stream(stream);
     LdePlan pl;
     if ((rc = get_plan(logn, le, plan_offset(trace_offset, extended_offset), &pl))) return rc;
     uint64_t* d_add = nullptr;
@@ -999,9 +1070,17 @@ int tvmc_lde_randomized_gpu(const uint64_t* d_traces, size_t num_columns, size_t
     rc = build_rand_add(d_randomizers, num_randomizers, num_columns, logn, le, trace_offset, extended_offset,
                         flags & TVMC_RAND_TRUNCATE, st, &d_add, &ra);
     if (rc) return rc;
-    rc = run_lde(pl, d_traces, trace_len, d_extended, extended_len, num_columns, st, ra);
+    rc = run_lde(pl, d_traces, trace_len, d_extended, extended_len, num_columns, st, status, ra);
     if (d_add) cudaFreeAsync(d_add, st);
     return rc;
+}
+
+int tvmc_lde_randomized_gpu(const uint64_t* d_traces, size_t num_columns, size_t trace_len,
+                            const uint64_t* d_randomizers, size_t num_randomizers, uint64_t* d_extended,
+                            size_t extended_len, uint64_t trace_offset, uint64_t extended_offset, uint32_t flags,
+                            void* stream) {
+    return lde_randomized_impl(d_traces, num_columns, trace_len, d_randomizers, num_randomizers, d_extended,
+                               extended_len, trace_offset, extended_offset, flags, as_stream(stream), nullptr);
 }
 
 int tvmc_lde_randomized_host(const uint64_t* traces, size_t num_columns, size_t trace_len,
@@ -1018,11 +1097,13 @@ int tvmc_lde_randomized_host(const uint64_t* traces, size_t num_columns, size_t 
     CK(r.alloc(num_randomizers * num_columns));
     CK(cudaMemcpy(a.p, traces, trace_len * num_columns * 8, cudaMemcpyHostToDevice));
     if (num_randomizers) CK(cudaMemcpy(r.p, randomizers, num_randomizers * num_columns * 8, cudaMemcpyHostToDevice));
-    rc = tvmc_lde_randomized_gpu(a.p, num_columns, trace_len, r.p, num_randomizers, b.p, extended_len, trace_offset,
-                                 extended_offset, flags, nullptr);
+    uint64_t* status = nullptr;
+    if ((rc = clear_status(&status))) return rc;
+    rc = lde_randomized_impl(a.p, num_columns, trace_len, r.p, num_randomizers, b.p, extended_len, trace_offset,
+                             extended_offset, flags, nullptr, status);
     if (rc) return rc;
     CK(cudaMemcpy(extended, b.p, extended_len * num_columns * 8, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
 // ---------------------------------------------------------------- Tip5
@@ -1030,7 +1111,7 @@ int tvmc_lde_randomized_host(const uint64_t* traces, size_t num_columns, size_t 
 int tvmc_hash_bfield_rows_gpu(const uint64_t* d_table, size_t num_rows, size_t num_cols, uint64_t* d_digests,
                               void* stream) {
     CK(launch_hash_rows(d_table, 1, num_rows, num_rows, (uint32_t)num_cols, d_digests, nullptr, LAYOUT_HEAP,
-                        as_stream(stream)));
+                        as_stream(stream), nullptr));
     return TVMC_OK;
 }
 
@@ -1045,14 +1126,16 @@ int tvmc_hash_varlen_host(const uint64_t* rows, size_t num_rows, size_t row_len,
     CK(a.alloc(num_rows * row_len));
     CK(b.alloc(num_rows * 5));
     if (row_len) CK(cudaMemcpy(a.p, rows, num_rows * row_len * 8, cudaMemcpyHostToDevice));
-    CK(launch_hash_rows(a.p, row_len, 1, num_rows, (uint32_t)row_len, b.p, nullptr, LAYOUT_HEAP, nullptr));
+    uint64_t* status = nullptr;
+    if (int rc = clear_status(&status)) return rc;
+    CK(launch_hash_rows(a.p, row_len, 1, num_rows, (uint32_t)row_len, b.p, nullptr, LAYOUT_HEAP, nullptr, status));
     CK(cudaMemcpy(digests, b.p, num_rows * 40, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
 int tvmc_hash_pairs_gpu(const uint64_t* d_left, const uint64_t* d_right, uint64_t* d_out, size_t count,
                         void* stream) {
-    CK(launch_hash_pairs(d_left, d_right, d_out, count, as_stream(stream)));
+    CK(launch_hash_pairs(d_left, d_right, d_out, count, as_stream(stream), nullptr));
     return TVMC_OK;
 }
 
@@ -1061,28 +1144,31 @@ int tvmc_hash_pairs_host(const uint64_t* left, const uint64_t* right, uint64_t* 
     HostBuf hb;
     int rc = host_buf(15 * count, &hb);
     if (rc) return rc;
-    uint64_t *a = hb.p, *b = a + 5 * count, *c = b + 5 * count;
+    uint64_t *a = hb.p, *b = a + 5 * count, *c = b + 5 * count, *status = nullptr;
+    if ((rc = clear_status(&status))) return rc;
     CK(cudaMemcpy(a, left, 40 * count, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b, right, 40 * count, cudaMemcpyHostToDevice));
-    CK(launch_hash_pairs(a, b, c, count, nullptr));
+    CK(launch_hash_pairs(a, b, c, count, nullptr, status));
     CK(cudaMemcpy(out, c, 40 * count, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
 int tvmc_tip5_permutation_batch_gpu(uint64_t* d_states, size_t num_states, void* stream) {
-    CK(launch_tip5_permutations(d_states, num_states, as_stream(stream)));
+    CK(launch_tip5_permutations(d_states, num_states, as_stream(stream), nullptr));
     return TVMC_OK;
 }
 
 int tvmc_tip5_permutation_batch_host(uint64_t* states, size_t num_states) {
     if (num_states == 0) return TVMC_OK;
     HostBuf a;
+    uint64_t* status = nullptr;
     int rc = host_buf(16 * num_states, &a);
+    if (!rc) rc = clear_status(&status);
     if (rc) return rc;
     CK(cudaMemcpy(a.p, states, 128 * num_states, cudaMemcpyHostToDevice));
-    CK(launch_tip5_permutations(a.p, num_states, nullptr));
+    CK(launch_tip5_permutations(a.p, num_states, nullptr, status));
     CK(cudaMemcpy(states, a.p, 128 * num_states, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
 int tvmc_tip5_rounds_host(uint64_t* states, size_t num_states, uint32_t first_round, uint32_t num_rounds,
@@ -1119,7 +1205,7 @@ int tvmc_tip5_parameters(uint8_t* lookup_table, uint64_t* mds_first_column, uint
 int tvmc_merkle_tree_gpu(const uint64_t* d_leaves, uint64_t* d_tree, size_t num_leaves, void* stream) {
     if (!is_pow2(num_leaves))
         return fail(TVMC_ERR_INVALID, "Number of leaves must be a power of 2 (got %zu)", num_leaves);
-    CK(launch_merkle_tree(d_leaves, d_tree, num_leaves, LAYOUT_FLAT, as_stream(stream)));
+    CK(launch_merkle_tree(d_leaves, d_tree, num_leaves, LAYOUT_FLAT, as_stream(stream), nullptr));
     return TVMC_OK;
 }
 
@@ -1129,7 +1215,7 @@ int tvmc_merkle_root_gpu(const uint64_t* d_leaves, uint64_t* d_root, size_t num_
     cudaStream_t st = as_stream(stream);
     uint64_t* tree = nullptr;
     CK(dev_malloc_async((void**)&tree, (2 * num_leaves - 1) * 40, st));
-    cudaError_t e = launch_merkle_tree(d_leaves, tree, num_leaves, LAYOUT_FLAT, st);
+    cudaError_t e = launch_merkle_tree(d_leaves, tree, num_leaves, LAYOUT_FLAT, st, nullptr);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_root, tree + 5 * (2 * num_leaves - 2), 40, cudaMemcpyDeviceToDevice, st);
     cudaFreeAsync(tree, st);
@@ -1168,9 +1254,11 @@ int tvmc_merkle_tree_heap_host(const uint64_t* leaves, size_t num_leaves, uint64
     CK(t.alloc(10 * num_leaves));
     CK(cudaMemcpy(a.p, leaves, 40 * num_leaves, cudaMemcpyHostToDevice));
     CK(cudaMemset(t.p, 0, 40));
-    CK(launch_merkle_tree(a.p, t.p, num_leaves, LAYOUT_HEAP, nullptr));
+    uint64_t* status = nullptr;
+    if (int rc = clear_status(&status)) return rc;
+    CK(launch_merkle_tree(a.p, t.p, num_leaves, LAYOUT_HEAP, nullptr, status));
     CK(cudaMemcpy(nodes, t.p, 80 * num_leaves, cudaMemcpyDeviceToHost));
-    return TVMC_OK;
+    return check_status(status);
 }
 
 // ---------------------------------------------------------------- commitment
@@ -1275,7 +1363,7 @@ int tvmc_commit_randomized(const uint64_t* trace, size_t trace_len, size_t width
         // host column-major trace: upload column chunks on a copy stream,
         // overlapping the LDE of the previous chunk
         if (prof) cudaEventRecord(c->prof[1], st);
-        rc = upload_lde_pipelined(pl, trace, trace_len, width, c->d_lde, c->L, st, ra);
+        rc = upload_lde_pipelined(pl, trace, trace_len, width, c->d_lde, c->L, st, c->d_nodes, ra);
         if (rc) return bail(rc);
     } else if (width) {
         const uint64_t* d_src = trace;
@@ -1298,7 +1386,7 @@ int tvmc_commit_randomized(const uint64_t* trace, size_t trace_len, size_t width
             return bail(cuda_fail(e, "trace upload"));
         }
         if (prof) cudaEventRecord(c->prof[1], st);
-        rc = run_lde(pl, d_src, trace_len, c->d_lde, c->L, width, st, ra);
+        rc = run_lde(pl, d_src, trace_len, c->d_lde, c->L, width, st, c->d_nodes, ra);
         if (d_up) cudaFreeAsync(d_up, st);
         if (d_cm) cudaFreeAsync(d_cm, st);
         if (rc) return bail(rc);
@@ -1307,8 +1395,8 @@ int tvmc_commit_randomized(const uint64_t* trace, size_t trace_len, size_t width
     }
     if (prof && !frugal) cudaEventRecord(c->prof[2], st);
     if (!frugal) {  // (the frugal stripes already hashed every row and built the tree)
-        cudaError_t e =
-            launch_hash_rows(c->d_lde, 1, c->L, c->L, (uint32_t)width, nullptr, c->d_nodes, LAYOUT_HEAP, st);
+        cudaError_t e = launch_hash_rows(c->d_lde, 1, c->L, c->L, (uint32_t)width, nullptr, c->d_nodes, LAYOUT_HEAP, st,
+                                         c->d_nodes);
         if (e != cudaSuccess) return bail(cuda_fail(e, "hash/merkle"));
     }
     if (prof) cudaEventRecord(c->prof[3], st);
@@ -1323,6 +1411,7 @@ int tvmc_commit_randomized(const uint64_t* trace, size_t trace_len, size_t width
     }
     if (flags & TVMC_SYNC) {
         if (cudaError_t e = cudaEventSynchronize(c->done); e != cudaSuccess) return bail(cuda_fail(e, "sync"));
+        if ((rc = wait_sound(c))) return bail(rc);
     }
     *out = c;
     return TVMC_OK;
@@ -1396,7 +1485,7 @@ int tvmc_commit_multi(const tvmc_multi_table* tables, size_t count, uint32_t fla
                     return bail(cuda_fail(e, "trace upload"));
                 src = d;
             }
-            if ((rc = run_lde(plans[i], src, t.trace_len, lde, c->L, t.width, st))) return bail(rc);
+            if ((rc = run_lde(plans[i], src, t.trace_len, lde, c->L, t.width, st, c->d_nodes))) return bail(rc);
         }
         hjobs.push_back(MultiHashTable{lde, c->d_nodes, c->L, (uint32_t)t.width});
     }
@@ -1409,6 +1498,8 @@ int tvmc_commit_multi(const tvmc_multi_table* tables, size_t count, uint32_t fla
     }
     if (flags & TVMC_SYNC) {
         if (cudaError_t e = cudaEventSynchronize(cs[count - 1]->done); e != cudaSuccess) return bail(cuda_fail(e, "sync"));
+        for (auto* c : cs)
+            if ((rc = wait_sound(c))) return bail(rc);
     }
     for (size_t i = 0; i < count; i++) out[i] = cs[i];
     return TVMC_OK;
@@ -1427,6 +1518,12 @@ static int finish_commitment(tvmc_commitment* c, uint32_t flags, tvmc_commitment
         const int rc = cuda_fail(e, "sync");
         tvmc_commitment_free(c);
         return rc;
+    }
+    if (flags & TVMC_SYNC) {
+        if (const int rc = wait_sound(c)) {
+            tvmc_commitment_free(c);
+            return rc;
+        }
     }
     *out = c;
     return TVMC_OK;
@@ -1478,7 +1575,8 @@ int tvmc_commit_rows(const uint64_t* table, size_t num_rows, size_t width, uint3
         if (e != cudaSuccess) return bail(cuda_fail(e, "row upload"));
         src = c->d_lde;
     }
-    cudaError_t e = launch_hash_rows(src, 1, num_rows, num_rows, (uint32_t)width, nullptr, c->d_nodes, LAYOUT_HEAP, st);
+    cudaError_t e = launch_hash_rows(src, 1, num_rows, num_rows, (uint32_t)width, nullptr, c->d_nodes, LAYOUT_HEAP, st,
+                                     c->d_nodes);
     if (e != cudaSuccess) return bail(cuda_fail(e, "hash/merkle"));
     if (discard && c->d_lde) {
         cudaFreeAsync(c->d_lde, st);
@@ -1521,7 +1619,7 @@ int tvmc_commit_digests(const uint64_t* leaves, size_t num_leaves, uint32_t flag
         if (e == cudaSuccess) e = cudaMemcpyAsync(up, leaves, num_leaves * words * 8, cudaMemcpyHostToDevice, st);
         src = up;
     }
-    if (e == cudaSuccess) e = launch_merkle_tree(src, c->d_nodes, num_leaves, LAYOUT_HEAP, st, words);
+    if (e == cudaSuccess) e = launch_merkle_tree(src, c->d_nodes, num_leaves, LAYOUT_HEAP, st, c->d_nodes, words);
     if (up) cudaFreeAsync(up, st);
     if (e != cudaSuccess) return bail(cuda_fail(e, "merkle"));
     return finish_commitment(c, flags, out);
@@ -1553,16 +1651,12 @@ int tvmc_commitment_absorb_root(tvmc_commitment* c, uint64_t* d_state, void* str
 int tvmc_commitment_sync(tvmc_commitment* c) {
     if (!c) return fail(TVMC_ERR_INVALID, "null handle");
     CK(cudaEventSynchronize(c->done));
-    return TVMC_OK;
+    return wait_sound(c);
 }
 
 int tvmc_commitment_root(tvmc_commitment* c, uint64_t* root) {
     if (!c || !root) return fail(TVMC_ERR_INVALID, "null argument");
-    uint64_t head[10];  // node 0 is zero unless a kernel of this commitment gave up waiting
-    if (int rc = read_sync(c, c->d_nodes, 10, head)) return rc;
-    if (head[0]) return fail(TVMC_ERR_TIMEOUT, "a device wait of this commitment ran out");
-    std::memcpy(root, head + 5, 40);
-    return TVMC_OK;
+    return wait_sound(c, root);
 }
 
 int tvmc_commitment_shape(const tvmc_commitment* c, size_t* lde_len, size_t* width) {
@@ -1640,6 +1734,7 @@ int tvmc_commitment_read_columns(tvmc_commitment* c, size_t col0, size_t ncols, 
         return fail(TVMC_ERR_RANGE, "columns [%zu, %zu) out of range", col0, col0 + ncols);
     if (ncols == 0) return TVMC_OK;
     CK(cudaEventSynchronize(c->done));
+    if (int rc = wait_sound(c)) return rc;
     CK(cudaMemcpy(out, c->d_lde + col0 * c->L, ncols * c->L * 8, cudaMemcpyDeviceToHost));
     return TVMC_OK;
 }
@@ -1649,6 +1744,7 @@ int tvmc_commitment_read_lde(tvmc_commitment* c, uint64_t* out, int row_major) {
     if (!c->d_lde && c->width) return fail(TVMC_ERR_INVALID, "LDE was discarded");
     if (c->width == 0) return TVMC_OK;
     CK(cudaEventSynchronize(c->done));
+    if (int rc = wait_sound(c)) return rc;
     const size_t W = c->L * c->width;
     if (!row_major) {
         CK(cudaMemcpy(out, c->d_lde, W * 8, cudaMemcpyDeviceToHost));
@@ -1797,10 +1893,12 @@ int tvmc_batch_create(const tvmc_table_shape* shapes, size_t count, tvmc_batch**
             e = cudaMemsetAsync(c->d_nodes, 0, 40, st);
             for (size_t c0 = 0; c0 < W && e == cudaSuccess; c0 += chunk[i]) {
                 const size_t nc = std::min(chunk[i], W - c0);
-                e = launch_lde(plans[i], b->inputs[i] + c0 * N, N, c->d_lde + c0 * c->L, c->L, nc, b->scratch[w], st);
+                e = launch_lde(plans[i], b->inputs[i] + c0 * N, N, c->d_lde + c0 * c->L, c->L, nc, b->scratch[w], st,
+                               c->d_nodes);
             }
             if (e == cudaSuccess && !multi)
-                e = launch_hash_rows(c->d_lde, 1, c->L, c->L, (uint32_t)W, nullptr, c->d_nodes, LAYOUT_HEAP, st);
+                e = launch_hash_rows(c->d_lde, 1, c->L, c->L, (uint32_t)W, nullptr, c->d_nodes, LAYOUT_HEAP, st,
+                                     c->d_nodes);
         }
         if (e == cudaSuccess) e = cudaEventRecord(b->events[w + 1], st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->capture, b->events[w + 1], 0);
@@ -1842,6 +1940,7 @@ int tvmc_batch_run(tvmc_batch* b, void* stream) {
     g_launches.fetch_add(b->kernels_per_run);
     for (auto* c : b->tables) {
         c->stream = st;
+        c->sound = false;
         CK(cudaEventRecord(c->done, st));
     }
     return TVMC_OK;

@@ -98,12 +98,13 @@ static inline unsigned grid_for(uint64_t work, unsigned threads) {
 
 // The m nodes of one level (heap indices [m, 2m)) of a tree with n leaves are
 // in place: build every level above.
-static cudaError_t launch_tree_above(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st) {
+static cudaError_t launch_tree_above(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st,
+                                     uint64_t* status) {
     while (m > 1) {
         int levels = 1;
         cudaError_t e;
         if ((m >> 1) >= MMA_MIN_PARENTS) {
-            e = launch_merkle_level_mma(tree, n, m, layout, st);
+            e = launch_merkle_level_mma(tree, n, m, layout, st, status);
         } else {
             levels = ilog2u(m) < COOP_TREE_LEVELS ? ilog2u(m) : COOP_TREE_LEVELS;
             e = launch_merkle_coop(tree, n, m, layout, levels, st);
@@ -114,19 +115,16 @@ static cudaError_t launch_tree_above(uint64_t* tree, uint64_t n, uint64_t m, int
     return cudaSuccess;
 }
 
-cudaError_t launch_merkle_from_leaves(uint64_t* tree, uint64_t n, int layout, cudaStream_t st) {
-    return launch_tree_above(tree, n, n, layout, st);  // n leaves already in place
-}
-
 cudaError_t launch_hash_rows(const uint64_t* table, uint64_t rstride, uint64_t cstride, uint64_t rows,
                              uint32_t width, uint64_t* digests, uint64_t* tree, int layout,
-                             cudaStream_t st) {
+                             cudaStream_t st, uint64_t* status) {
     if (rows == 0) return cudaSuccess;
     NvtxRange range("tvmc row hash + Merkle tree");
     const cudaError_t e =
         rows <= COOP_MAX_ROWS ? launch_hash_rows_coop(table, rstride, cstride, rows, width, digests, tree, layout, st)
-                              : launch_hash_rows_mma(table, rstride, cstride, rows, width, digests, tree, layout, st);
-    return e != cudaSuccess || !tree ? e : launch_tree_above(tree, rows, rows, layout, st);
+                              : launch_hash_rows_mma(table, rstride, cstride, rows, width, digests, tree, layout, st,
+                                                     status);
+    return e != cudaSuccess || !tree ? e : launch_tree_above(tree, rows, rows, layout, st, status);
 }
 
 // Every level above the leaves of each of count heap trees, all trees in each
@@ -180,25 +178,25 @@ cudaError_t launch_hash_rows_multi(const MultiHashTable* tabs, int count, cudaSt
 }
 
 cudaError_t launch_merkle_tree(const uint64_t* leaves, uint64_t* tree, uint64_t n, int layout,
-                               cudaStream_t st, int leaf_words) {
+                               cudaStream_t st, uint64_t* status, int leaf_words) {
     count_launch();
     k_copy_leaves<<<grid_for(n, 256), 256, 0, st>>>(leaves, tree, n, layout, leaf_words);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return launch_merkle_from_leaves(tree, n, layout, st);
+    return launch_tree_above(tree, n, n, layout, st, status);
 }
 
 cudaError_t launch_hash_pairs(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
-                              cudaStream_t st) {
+                              cudaStream_t st, uint64_t* status) {
     if (count == 0) return cudaSuccess;
     return count < MMA_MIN_PARENTS ? launch_hash_pairs_coop(left, right, out, count, st)
-                                   : launch_hash_pairs_mma(left, right, out, count, st);
+                                   : launch_hash_pairs_mma(left, right, out, count, st, status);
 }
 
-cudaError_t launch_tip5_permutations(uint64_t* states, uint64_t count, cudaStream_t st) {
+cudaError_t launch_tip5_permutations(uint64_t* states, uint64_t count, cudaStream_t st, uint64_t* status) {
     if (count == 0) return cudaSuccess;
     return count < MMA_MIN_PARENTS ? launch_tip5_permutations_coop(states, count, st)
-                                   : launch_tip5_permutations_mma(states, count, st);
+                                   : launch_tip5_permutations_mma(states, count, st, status);
 }
 
 cudaError_t launch_tip5_rounds(uint64_t* states, uint64_t count, int r0, int nr, uint64_t* trace, cudaStream_t st) {
@@ -237,7 +235,7 @@ cudaError_t launch_absorb_stripe(const uint64_t* stripe, uint64_t L, uint32_t nc
                                  int last, uint64_t* tree, cudaStream_t st) {
     NvtxRange range("tvmc frugal stripe absorb");
     const cudaError_t e = launch_absorb_stripe_mma(stripe, L, ncols, cap, first, last, tree, st);
-    return e != cudaSuccess || !last ? e : launch_tree_above(tree, L, L, LAYOUT_HEAP, st);
+    return e != cudaSuccess || !last ? e : launch_tree_above(tree, L, L, LAYOUT_HEAP, st, tree);
 }
 
 }  // namespace tvmc

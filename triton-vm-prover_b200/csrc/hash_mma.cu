@@ -20,10 +20,8 @@ extern __shared__ uint8_t t5m_smem[];
 
 __device__ __forceinline__ uint32_t dyn_base() { return (uint32_t)__cvta_generic_to_shared(t5m_smem); }
 
-// Marks a commitment whose kernels timed out: word 0 of the heap tree's unused
-// node 0 (zero otherwise).
-__device__ __forceinline__ void mark_dead(const T5Mma& c, uint64_t* heap) {
-    if (c.waits.dead && heap) heap[0] = 1;
+__device__ __forceinline__ void mark_dead(const T5Mma& c, uint64_t* status) {
+    if (c.waits.dead && status) *status = 1;
 }
 
 // Absorbs `perms` chunks of the row at p (element i at p[i * cs]): its n
@@ -116,13 +114,12 @@ __device__ __forceinline__ void for_tiles(const T5Mma& c, const TileSpan& s, F&&
 
 }  // namespace
 
-// Leaf digests of `rows` rows, element (r, c) at tab[r * rstride + c * cstride]:
-// to tree leaf slots (tree non-null), else to digests.
+// Leaf digests of `rows` rows, element (r, c) at tab[r * rstride + c * cstride], to
+// consecutive slots (the leaves of a tree are, in either layout).
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_mma(const uint64_t* __restrict__ tab, uint64_t rstride,
                                                                   uint64_t cstride, uint64_t rows, uint32_t width,
-                                                                  uint64_t* __restrict__ digests,
-                                                                  uint64_t* __restrict__ tree, int layout,
-                                                                  TileSpan span) {
+                                                                  uint64_t* __restrict__ leaves,
+                                                                  uint64_t* status, TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
     for_tiles(c, span, [&](uint64_t tile) {
@@ -131,9 +128,9 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_rows_mma(const uint64_t
         uint64_t s[T5M_WORDS];
         zero(s);
         absorb(s, tab + (live ? row : 0) * rstride, cstride, width / T5_RATE + 1, width, c);
-        if (live) store_digest(s, tree ? tree + 5 * node_slot(rows + row, rows, layout) : digests + 5 * row, c);
+        if (live) store_digest(s, leaves + 5 * row, c);
     });
-    mark_dead(c, layout == LAYOUT_HEAP ? tree : nullptr);
+    mark_dead(c, status);
     t5m_done(c);
 }
 
@@ -200,7 +197,8 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_absorb_stripe_mma(const uint
 
 // One tree level: parent p in [m/2, m) = hash_pair(node 2p, node 2p + 1).
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_level_mma(uint64_t* __restrict__ tree, uint64_t n,
-                                                                     uint64_t m, int layout, TileSpan span) {
+                                                                     uint64_t m, int layout, uint64_t* status,
+                                                                     TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
     const uint64_t parents = m >> 1;
@@ -212,7 +210,7 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_level_mma(uint64_t* _
         pair_hash(s, tree + 5 * node_slot(2 * par, n, layout), tree + 5 * node_slot(2 * par + 1, n, layout), c);
         if (live) store_digest(s, tree + 5 * node_slot(par, n, layout), c);
     });
-    mark_dead(c, layout == LAYOUT_HEAP ? tree : nullptr);
+    mark_dead(c, status);
     t5m_done(c);
 }
 
@@ -240,7 +238,7 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_merkle_levels_mma(const __gr
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_pairs_mma(const uint64_t* __restrict__ left,
                                                                    const uint64_t* __restrict__ right,
                                                                    uint64_t* __restrict__ out, uint64_t count,
-                                                                   TileSpan span) {
+                                                                   uint64_t* status, TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
     for_tiles(c, span, [&](uint64_t tile) {
@@ -249,11 +247,12 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_hash_pairs_mma(const uint64_
         pair_hash(s, left + 5 * k, right + 5 * k, c);
         if (i < count) store_digest(s, out + 5 * i, c);
     });
+    mark_dead(c, status);
     t5m_done(c);
 }
 
 __global__ void __launch_bounds__(T5M_THREADS, 1) k_tip5_perm_mma(uint64_t* __restrict__ states, uint64_t count,
-                                                                  TileSpan span) {
+                                                                  uint64_t* status, TileSpan span) {
     T5Mma c;
     t5m_init(c, dyn_base());
     for_tiles(c, span, [&](uint64_t tile) {
@@ -269,14 +268,16 @@ __global__ void __launch_bounds__(T5M_THREADS, 1) k_tip5_perm_mma(uint64_t* __re
             for (int k = 0; k < T5M_WORDS; k++) states[T5_STATE * i + t5m_word(c.part, k)] = gl_from_mont(s[k]);
         }
     });
+    mark_dead(c, status);
     t5m_done(c);
 }
 
 namespace {
 
-// kern(args..., span) over tiles of perms permutations each.
+// kern(args..., span) over tiles of perms permutations each; status: the (first)
+// word it reports to.
 template <class... P, class... A>
-cudaError_t launch(void (*kern)(P...), uint64_t tiles, uint64_t perms, cudaStream_t st, A... args) {
+cudaError_t launch(void (*kern)(P...), uint64_t tiles, uint64_t perms, cudaStream_t st, uint64_t* status, A... args) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -285,7 +286,7 @@ cudaError_t launch(void (*kern)(P...), uint64_t tiles, uint64_t perms, cudaStrea
     const TileSpan span = tile_span(tiles, perms, sms);
     count_launch();
     kern<<<span_ctas(span), T5M_THREADS, T5M_BYTES, st>>>(args..., span);
-    return cudaGetLastError();
+    return mma_launched(status, st);
 }
 
 }  // namespace
@@ -293,36 +294,39 @@ cudaError_t launch(void (*kern)(P...), uint64_t tiles, uint64_t perms, cudaStrea
 uint64_t mma_tiles(uint64_t rows) { return (rows + T5M_STATES - 1) / T5M_STATES; }
 
 cudaError_t launch_hash_rows_mma(const uint64_t* table, uint64_t rstride, uint64_t cstride, uint64_t rows,
-                                 uint32_t width, uint64_t* digests, uint64_t* tree, int layout, cudaStream_t st) {
-    return launch(k_hash_rows_mma, mma_tiles(rows), width / T5_RATE + 1, st, table, rstride, cstride, rows, width, digests, tree, layout);
+                                 uint32_t width, uint64_t* digests, uint64_t* tree, int layout, cudaStream_t st,
+                                 uint64_t* status) {
+    return launch(k_hash_rows_mma, mma_tiles(rows), width / T5_RATE + 1, st, status, table, rstride, cstride, rows, width,
+                  tree ? tree + 5 * node_slot(rows, rows, layout) : digests, status);
 }
 
 cudaError_t launch_hash_jobs_mma(const HashJobs& jobs, uint32_t tiles, cudaStream_t st) {
     uint32_t width = 0;
     for (int k = 0; k < jobs.count; k++) width = jobs.j[k].width > width ? jobs.j[k].width : width;
-    return launch(k_hash_rows_multi_mma, tiles, width / T5_RATE + 1, st, jobs);
+    return launch(k_hash_rows_multi_mma, tiles, width / T5_RATE + 1, st, jobs.j[0].tree, jobs);
 }
 
 cudaError_t launch_absorb_stripe_mma(const uint64_t* stripe, uint64_t L, uint32_t ncols, uint64_t* cap, int first,
                                      int last, uint64_t* tree, cudaStream_t st) {
-    return launch(k_absorb_stripe_mma, mma_tiles(L), ncols / T5_RATE + 1, st, stripe, L, ncols, cap, first, last, tree);
+    return launch(k_absorb_stripe_mma, mma_tiles(L), ncols / T5_RATE + 1, st, tree, stripe, L, ncols, cap, first, last, tree);
 }
 
-cudaError_t launch_merkle_level_mma(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st) {
-    return launch(k_merkle_level_mma, mma_tiles(m >> 1), 1, st, tree, n, m, layout);
+cudaError_t launch_merkle_level_mma(uint64_t* tree, uint64_t n, uint64_t m, int layout, cudaStream_t st,
+                                    uint64_t* status) {
+    return launch(k_merkle_level_mma, mma_tiles(m >> 1), 1, st, status, tree, n, m, layout, status);
 }
 
 cudaError_t launch_merkle_levels_mma(const LevelJobs& jobs, uint32_t tiles, cudaStream_t st) {
-    return launch(k_merkle_levels_mma, tiles, 1, st, jobs);
+    return launch(k_merkle_levels_mma, tiles, 1, st, jobs.j[0].tree, jobs);
 }
 
 cudaError_t launch_hash_pairs_mma(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
-                                  cudaStream_t st) {
-    return launch(k_hash_pairs_mma, mma_tiles(count), 1, st, left, right, out, count);
+                                  cudaStream_t st, uint64_t* status) {
+    return launch(k_hash_pairs_mma, mma_tiles(count), 1, st, status, left, right, out, count, status);
 }
 
-cudaError_t launch_tip5_permutations_mma(uint64_t* states, uint64_t count, cudaStream_t st) {
-    return launch(k_tip5_perm_mma, mma_tiles(count), 1, st, states, count);
+cudaError_t launch_tip5_permutations_mma(uint64_t* states, uint64_t count, cudaStream_t st, uint64_t* status) {
+    return launch(k_tip5_perm_mma, mma_tiles(count), 1, st, status, states, count, status);
 }
 
 unsigned int mma_timeouts() {

@@ -70,6 +70,16 @@ __host__ __device__ inline uint64_t node_slot(uint64_t h, uint64_t n, int layout
     return 2 * n + h - 3 * pm;
 }
 
+// ---- device waits ---------------------------------------------------------
+// A kernel whose waits are bounded (the tensor-core forms) goes on after one ran
+// out and leaves a wrong result.  Launchers take `status`, a device-visible word
+// that such a kernel sets to 1: node 0 of the heap tree for a commitment's kernels
+// (zero otherwise), a host word for the calls that return host data; null where
+// the caller has device pointers only ("mma_timeouts" then still counts it).
+// Every tensor-core launch ends with this: cudaGetLastError(), and, for tests of
+// what follows (tuning key "fail_mma_after"), *status set as by a wait that ran out.
+cudaError_t mma_launched(uint64_t* status, cudaStream_t st);
+
 // ---- hash.cu -------------------------------------------------------------
 // Leaf digests of `rows` rows; element (r, c) at table[r*rstride + c*cstride].
 // If `tree` is non-null, rows must be a power of two: leaves are written as
@@ -77,20 +87,19 @@ __host__ __device__ inline uint64_t node_slot(uint64_t h, uint64_t n, int layout
 // Otherwise digests go to `digests` (rows x 5).
 cudaError_t launch_hash_rows(const uint64_t* table, uint64_t rstride, uint64_t cstride, uint64_t rows,
                              uint32_t width, uint64_t* digests, uint64_t* tree, int layout,
-                             cudaStream_t st);
-// Complete a tree whose leaf level (n leaves) is already stored in `tree`.
-cudaError_t launch_merkle_from_leaves(uint64_t* tree, uint64_t n, int layout, cudaStream_t st);
+                             cudaStream_t st, uint64_t* status);
 // Copy n leaf digests into the tree's leaf slots and complete the tree.  With
 // leaf_words = 3 the leaves are XFieldElements, each padded to (c0, c1, c2, 0, 0).
 cudaError_t launch_merkle_tree(const uint64_t* leaves, uint64_t* tree, uint64_t n, int layout,
-                               cudaStream_t st, int leaf_words = 5);
+                               cudaStream_t st, uint64_t* status, int leaf_words = 5);
 // Frugal streaming: absorb ncols LDE columns (stride L) into per-row capacity
 // state cap[6][L]; `last` pads, finishes the digests as leaves of the heap tree
-// (2L digests) and builds the whole tree.
+// (2L digests) and builds the whole tree.  The status word is the tree's node 0, here
+// and in launch_hash_rows_multi.
 cudaError_t launch_absorb_stripe(const uint64_t* stripe, uint64_t L, uint32_t ncols, uint64_t* cap, int first,
                                  int last, uint64_t* tree, cudaStream_t st);
 cudaError_t launch_hash_pairs(const uint64_t* left, const uint64_t* right, uint64_t* out, uint64_t count,
-                              cudaStream_t st);
+                              cudaStream_t st, uint64_t* status);
 
 // Multi-table row hash + heap Merkle trees: every launch takes all of up to
 // HASH_MULTI_MAX tables, the rows first and then the trees' levels.
@@ -122,7 +131,7 @@ struct LevelJobs {
     int count;
 };
 cudaError_t launch_hash_rows_multi(const MultiHashTable* tabs, int count, cudaStream_t st);
-cudaError_t launch_tip5_permutations(uint64_t* states, uint64_t count, cudaStream_t st);
+cudaError_t launch_tip5_permutations(uint64_t* states, uint64_t count, cudaStream_t st, uint64_t* status);
 // Fiat-Shamir absorb of [lead (if has_lead)] ++ data[0..len) into the 16-word sponge state.
 cudaError_t launch_sponge_absorb(uint64_t* state, const uint64_t* data, uint64_t len, int has_lead, uint64_t lead,
                                  cudaStream_t st);
@@ -164,8 +173,8 @@ struct LdePlan {
 // these columns ([col][coset][rm]); the plan's offset is then o / t.
 size_t lde_scratch_words(int logn, int log_exp, uint64_t cols);
 cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, uint64_t* out, uint64_t old,
-                       uint64_t cols, uint64_t* scratch, cudaStream_t st, const uint64_t* add = nullptr,
-                       int rm = 0);
+                       uint64_t cols, uint64_t* scratch, cudaStream_t st, uint64_t* status,
+                       const uint64_t* add = nullptr, int rm = 0);
 // The same for trace lengths 2^1 .. 2^11: whole columns per CTA, no scratch.
 cudaError_t launch_lde_small(const LdePlan& pl, const uint64_t* trace, uint64_t tld, uint64_t* out, uint64_t old,
                              uint64_t cols, const uint64_t* add, int rm, cudaStream_t st);
@@ -182,7 +191,7 @@ cudaError_t launch_rand_addend(const uint64_t* r, uint64_t R, uint64_t cols, int
 // Batched NTT in place on column-major data[c*ld + r], r < 2^logn.
 size_t ntt_scratch_words(int logn, uint64_t cols);
 cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t ld, uint64_t cols,
-                       uint64_t* scratch, cudaStream_t st);
+                       uint64_t* scratch, cudaStream_t st, uint64_t* status);
 // out[c*L + i] = in[c*ild + i] * o^i for i < min(n, L), 0 above (the coefficient
 // side of NTT::evaluate_on_coset); a forward NTT of length L finishes it.
 cudaError_t launch_coset_scale(const uint64_t* in, uint64_t ild, uint64_t n, uint64_t* out, uint64_t L, uint64_t cols,

@@ -146,9 +146,10 @@ __device__ __forceinline__ void lm_init(Lm& c, const uint64_t* tw12) {
     c.waits = GroupWaits{};
 }
 
-// Every thread of the CTA calls this last.
+// Every thread of the CTA calls this last; sets *status if a wait ran out.
 template <int B>
-__device__ __forceinline__ void lm_done(const Lm& c) {
+__device__ __forceinline__ void lm_done(const Lm& c, uint64_t* status) {
+    if (c.waits.dead && status) *status = 1;
     if ((threadIdx.x & (LmCfg<B>::GROUP - 1)) == 0) mma8_drain(c.bar, c.waits);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -273,7 +274,7 @@ template <int B, bool INV>
 __global__ void __launch_bounds__(LM_THREADS, 1) k_pass_a_mma(const uint64_t* __restrict__ in, uint64_t ild,
                                                               uint64_t* __restrict__ Y, uint64_t yld, uint32_t cols,
                                                               uint32_t unit, int l1, const uint64_t* tw12, const uint64_t* wlo,
-                                                              const uint64_t* whi) {
+                                                              const uint64_t* whi, uint64_t* status) {
     using C = LmCfg<B>;
     Lm c;
     lm_init<B>(c, tw12);
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_pass_a_mma(const uint64_t* __
             dst += (uint64_t)(8 * C::R * c.part + d) << l1;
             lm_store<B>(c, dst, l1, [&](int i, uint64_t x) { return gl_mont_mul(x, twq[128 * i]); });
         });
-    lm_done<B>(c);
+    lm_done<B>(c, status);
 }
 
 // K2: rows k2 of Y (R*R points): inverse DFT -> coefficients; per coset c: times
@@ -307,7 +308,8 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_lde_mid_mma(const uint64_t* _
                                                                const uint64_t* tw12, const uint64_t* wlo,
                                                                const uint64_t* whi, const uint64_t* sc_lo,
                                                                const uint64_t* sc_hi, int hi_len,
-                                                               const uint64_t* __restrict__ add, int rm) {
+                                                               const uint64_t* __restrict__ add, int rm,
+                                                               uint64_t* status) {
     using C = LmCfg<B>;
     Lm c;
     lm_init<B>(c, tw12);
@@ -363,7 +365,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_lde_mid_mma(const uint64_t* _
                 lm_store<B>(c, dst, l2, [&](int i, uint64_t x) { return gl_mont_mul(x, twq[128 * i]); });
             }
         });
-    lm_done<B>(c);
+    lm_done<B>(c, status);
 }
 
 // K3, and pass B of the plain NTT: rows of R*R points, forward DFT (INV: inverse,
@@ -372,7 +374,8 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_lde_mid_mma(const uint64_t* _
 template <int B, bool INV>
 __global__ void __launch_bounds__(LM_THREADS, 1) k_pass_b_mma(const uint64_t* __restrict__ Z,
                                                               uint64_t* __restrict__ out, uint64_t old, uint32_t cols,
-                                                              int l1, int le, const uint64_t* tw12, uint64_t scale) {
+                                                              int l1, int le, const uint64_t* tw12, uint64_t scale,
+                                                              uint64_t* status) {
     using C = LmCfg<B>;
     Lm c;
     lm_init<B>(c, tw12);
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_pass_b_mma(const uint64_t* __
                         ((uint64_t)(8 * C::R * c.part + d) << (l1 + le));
         lm_store<B>(c, dst, l1 + le, [&](int, uint64_t x) { return INV ? gl_mont_mul(x, scale) : x; });
     }
-    lm_done<B>(c);
+    lm_done<B>(c, status);
 }
 
 namespace {
@@ -410,15 +413,15 @@ int sm_count() {
     return sms;
 }
 
-// At most one CTA per SM.
+// kern(args..., status); at most one CTA per SM.
 template <class... P, class... A>
-cudaError_t launch(void (*kern)(P...), uint64_t work, uint32_t bytes, cudaStream_t st, A... args) {
+cudaError_t launch(void (*kern)(P...), uint64_t work, uint32_t bytes, cudaStream_t st, uint64_t* status, A... args) {
     const cudaError_t e = raise_smem_limit((const void*)kern);
     if (e != cudaSuccess) return e;
     const uint64_t sms = (uint64_t)sm_count();
     count_launch();
-    kern<<<(unsigned)(work < sms ? work : sms), LM_THREADS, bytes + LM_SLACK, st>>>(args...);
-    return cudaGetLastError();
+    kern<<<(unsigned)(work < sms ? work : sms), LM_THREADS, bytes + LM_SLACK, st>>>(args..., status);
+    return mma_launched(status, st);
 }
 
 // Columns per unit: sixteen, to share a block's tables widely, but fewer (down to
@@ -432,51 +435,51 @@ uint32_t unit_cols(uint64_t blocks, uint32_t cols) {
 
 template <int B>
 cudaError_t pass_a(const LdePlan& pl, bool inverse, const uint64_t* in, uint64_t ild, uint64_t* Y, uint64_t yld,
-                   uint32_t cols, int l1, cudaStream_t st) {
+                   uint32_t cols, int l1, cudaStream_t st, uint64_t* status) {
     using C = LmCfg<B>;
     const uint64_t blocks = (1u << l1) / C::SEQS;
     const uint32_t unit = unit_cols<B>(blocks, cols);
     return launch(inverse ? k_pass_a_mma<B, true> : k_pass_a_mma<B, false>, blocks * ((cols + unit - 1) / unit),
-                  C::BYTES, st, in, ild, Y, yld, cols, unit, l1, pl.tw12_f, inverse ? pl.wn_i_lo : pl.wn_f_lo,
+                  C::BYTES, st, status, in, ild, Y, yld, cols, unit, l1, pl.tw12_f, inverse ? pl.wn_i_lo : pl.wn_f_lo,
                   inverse ? pl.wn_i_hi : pl.wn_f_hi);
 }
 template <int B>
 cudaError_t mid(const LdePlan& pl, const uint64_t* Y, uint64_t yld, uint64_t* Z, uint32_t cols, int l2, int hi_len,
-                const uint64_t* add, int rm, cudaStream_t st) {
+                const uint64_t* add, int rm, cudaStream_t st, uint64_t* status) {
     using C = LmCfg<B>;
     const uint64_t blocks = (1u << l2) / C::SEQS;
     const uint32_t unit = unit_cols<B>(blocks, cols);
     return launch(rm ? k_lde_mid_mma<B, true> : k_lde_mid_mma<B, false>, blocks * ((cols + unit - 1) / unit),
-                  C::mid_bytes(pl.log_exp), st, Y, yld, Z, cols, unit, l2, pl.log_exp, pl.tw12_f, pl.wn_f_lo,
+                  C::mid_bytes(pl.log_exp), st, status, Y, yld, Z, cols, unit, l2, pl.log_exp, pl.tw12_f, pl.wn_f_lo,
                   pl.wn_f_hi, pl.sc_lo, pl.sc_hi, hi_len, add, rm);
 }
 template <int B>
 cudaError_t pass_b(const LdePlan& pl, bool inverse, const uint64_t* Z, uint64_t* out, uint64_t old, uint32_t cols,
-                   int l1, int le, uint64_t scale, cudaStream_t st) {
+                   int l1, int le, uint64_t scale, cudaStream_t st, uint64_t* status) {
     using C = LmCfg<B>;
     const uint64_t tiles = ((uint64_t)cols << (l1 + le)) / C::SEQS;
     return launch(inverse ? k_pass_b_mma<B, true> : k_pass_b_mma<B, false>, (tiles + C::GROUPS - 1) / C::GROUPS,
-                  C::BYTES, st, Z, out, old, cols, l1, le, pl.tw12_f, scale);
+                  C::BYTES, st, status, Z, out, old, cols, l1, le, pl.tw12_f, scale);
 }
 
 }  // namespace
 
 cudaError_t launch_pass_a_mma(int lsub, const LdePlan& pl, bool inverse, const uint64_t* in, uint64_t ild, uint64_t* Y,
-                              uint64_t yld, uint32_t cols, int l1, cudaStream_t st) {
-    return lsub == 10 ? pass_a<5>(pl, inverse, in, ild, Y, yld, cols, l1, st)
-                      : pass_a<4>(pl, inverse, in, ild, Y, yld, cols, l1, st);
+                              uint64_t yld, uint32_t cols, int l1, cudaStream_t st, uint64_t* status) {
+    return lsub == 10 ? pass_a<5>(pl, inverse, in, ild, Y, yld, cols, l1, st, status)
+                      : pass_a<4>(pl, inverse, in, ild, Y, yld, cols, l1, st, status);
 }
 
 cudaError_t launch_lde_mid_mma(int lsub, const LdePlan& pl, const uint64_t* Y, uint64_t yld, uint64_t* Z, uint32_t cols,
-                               int l2, int hi_len, const uint64_t* add, int rm, cudaStream_t st) {
-    return lsub == 10 ? mid<5>(pl, Y, yld, Z, cols, l2, hi_len, add, rm, st)
-                      : mid<4>(pl, Y, yld, Z, cols, l2, hi_len, add, rm, st);
+                               int l2, int hi_len, const uint64_t* add, int rm, cudaStream_t st, uint64_t* status) {
+    return lsub == 10 ? mid<5>(pl, Y, yld, Z, cols, l2, hi_len, add, rm, st, status)
+                      : mid<4>(pl, Y, yld, Z, cols, l2, hi_len, add, rm, st, status);
 }
 
 cudaError_t launch_pass_b_mma(int lsub, const LdePlan& pl, bool inverse, const uint64_t* Z, uint64_t* out, uint64_t old,
-                              uint32_t cols, int l1, int le, uint64_t scale_mont, cudaStream_t st) {
-    return lsub == 10 ? pass_b<5>(pl, inverse, Z, out, old, cols, l1, le, scale_mont, st)
-                      : pass_b<4>(pl, inverse, Z, out, old, cols, l1, le, scale_mont, st);
+                              uint32_t cols, int l1, int le, uint64_t scale_mont, cudaStream_t st, uint64_t* status) {
+    return lsub == 10 ? pass_b<5>(pl, inverse, Z, out, old, cols, l1, le, scale_mont, st, status)
+                      : pass_b<4>(pl, inverse, Z, out, old, cols, l1, le, scale_mont, st, status);
 }
 
 unsigned int lde_mma_timeouts() {

@@ -178,7 +178,7 @@ extern "C" int tvmc_lde_batch_noalloc_gpu(const uint64_t* d_traces, size_t num_c
     for (size_t c0 = 0; c0 < num_columns; c0 += chunk) {
         const size_t nc = num_columns - c0 < chunk ? num_columns - c0 : chunk;
         e = launch_lde(pl, d_traces + c0 * trace_len, trace_len, d_extended + c0 * extended_len, extended_len, nc,
-                       work, st);
+                       work, st, nullptr);
         if (e != cudaSuccess) return fail(TVMC_ERR_CUDA, "launch_lde: %s", cudaGetErrorString(e));
     }
     return TVMC_OK;

@@ -634,7 +634,7 @@ static int mma_split(int l) {
 size_t ntt_scratch_words(int logn, uint64_t cols) { return logn <= 11 ? 0 : (size_t)cols << logn; }
 
 cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t ld, uint64_t cols,
-                       uint64_t* scratch, cudaStream_t st) {
+                       uint64_t* scratch, cudaStream_t st, uint64_t* status) {
     const int l = pl.logn;
     const uint64_t* tw12 = pl.tw12_f;  // the inverse negates the sub-DFT input indices instead
     const uint64_t scale = (inverse && l > 0) ? GL_P - ((GL_P - 1) >> l) : 1;  // n^-1 = p - (p-1)/n
@@ -666,7 +666,7 @@ cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t 
     for (uint64_t c0 = 0; c0 < cols; c0 += 65535) {
         const unsigned nc = (unsigned)((cols - c0) < 65535 ? (cols - c0) : 65535);
         cudaError_t e = mma && lde_mma_size(l2)
-                            ? launch_pass_a_mma(l2, pl, inverse, data + c0 * ld, ld, scratch, n, nc, l1, st)
+                            ? launch_pass_a_mma(l2, pl, inverse, data + c0 * ld, ld, scratch, n, nc, l1, st, status)
                             : dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
             auto kern = inverse ? k_pass_a<L2, true> : k_pass_a<L2, false>;
             cudaError_t e2 = set_smem((const void*)kern, smem_a);
@@ -678,7 +678,7 @@ cudaError_t launch_ntt(const LdePlan& pl, int inverse, uint64_t* data, uint64_t 
         });
         if (e != cudaSuccess) return e;
         e = mma && lde_mma_size(l1)
-                ? launch_pass_b_mma(l1, pl, inverse, scratch, data + c0 * ld, ld, nc, l2, 0, scale_mont, st)
+                ? launch_pass_b_mma(l1, pl, inverse, scratch, data + c0 * ld, ld, nc, l2, 0, scale_mont, st, status)
                 : dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
             auto kern = inverse ? k_pass_b<L1, true> : k_pass_b<L1, false>;
             cudaError_t e2 = set_smem((const void*)kern, smem_b);
@@ -699,7 +699,8 @@ size_t lde_scratch_words(int logn, int log_exp, uint64_t cols) {
 }
 
 cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, uint64_t* out, uint64_t old,
-                       uint64_t cols, uint64_t* scratch, cudaStream_t st, const uint64_t* add, int rm) {
+                       uint64_t cols, uint64_t* scratch, cudaStream_t st, uint64_t* status, const uint64_t* add,
+                       int rm) {
     const int l = pl.logn, le = pl.log_exp;
     const int hi_len = l > 12 ? (1 << (l - 12)) : 1;
     if (cols == 0) return cudaSuccess;
@@ -741,7 +742,7 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
         const unsigned nc = (unsigned)((cols - c0) < 65535 ? (cols - c0) : 65535);
         uint64_t* Z = scratch + (size_t)nc * N;
         const uint64_t* addc = rm ? add + c0 * ((uint64_t)rm << le) : nullptr;
-        cudaError_t e = mma_ab ? launch_pass_a_mma(l2, pl, true, trace + c0 * tld, tld, Y, N, nc, l1, st)
+        cudaError_t e = mma_ab ? launch_pass_a_mma(l2, pl, true, trace + c0 * tld, tld, Y, N, nc, l1, st, status)
                                : dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
             cudaError_t e2 = set_smem((const void*)k_lde_inv_a<L2>, smem1);
             if (e2 != cudaSuccess) return e2;
@@ -751,7 +752,7 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
             return cudaGetLastError();
         });
         if (e != cudaSuccess) return e;
-        e = mma_mid ? launch_lde_mid_mma(l1, pl, Y, N, Z, nc, l2, hi_len, addc, rm, st)
+        e = mma_mid ? launch_lde_mid_mma(l1, pl, Y, N, Z, nc, l2, hi_len, addc, rm, st, status)
                     : dispatch_ls(l1, [&]<int L1>() -> cudaError_t {
             if constexpr (Plan<L1>::NR == 2 && Plan<L1>::b1 == Plan<L1>::b2) {
                 constexpr int lTr = 7 - Plan<L1>::b2;
@@ -802,7 +803,7 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
             return cudaGetLastError();
         });
         if (e != cudaSuccess) return e;
-        e = mma_ab ? launch_pass_b_mma(l2, pl, false, Z, out + c0 * old, old, nc, l1, le, 0, st)
+        e = mma_ab ? launch_pass_b_mma(l2, pl, false, Z, out + c0 * old, old, nc, l1, le, 0, st, status)
                    : dispatch_ls(l2, [&]<int L2>() -> cudaError_t {
             cudaError_t e2 = set_smem((const void*)k_lde_fwd_b<L2>, smem3);
             if (e2 != cudaSuccess) return e2;

@@ -414,7 +414,10 @@ int tvmc_server_wait(tvmc_server* s, uint64_t id, int64_t timeout_ms, uint64_t* 
     tvmc_commitment* c = r->c;
     lk.unlock();
     if (!c) return tvmc::set_error(TVMC_ERR_CUDA, "request finished without a commitment");
-    return root ? tvmc_commitment_root(c, root) : TVMC_OK;
+    const int rc = root ? tvmc_commitment_root(c, root) : tvmc_commitment_sync(c);
+    // the commit failed, which waiting longer does not mend
+    if (rc == TVMC_ERR_TIMEOUT) return tvmc::set_error(TVMC_ERR_CUDA, "a device wait of this request's commit ran out");
+    return rc;
 }
 
 int tvmc_server_open(tvmc_server* s, uint64_t id, const size_t* leaf_idx, size_t count, uint64_t* paths,
