@@ -1,0 +1,62 @@
+"""The tuner's cache and candidates, with the library's calls and the clock replaced
+(what it times on a GPU is the caller's business)."""
+import json
+
+import pytest
+
+import autotune
+
+SHAPE = dict(trace_len=1 << 20, width=379, expansion=4)
+
+
+@pytest.fixture
+def fake(monkeypatch, tmp_path):
+    """A tuner on a machine without a GPU: records the knobs set; every candidate takes 1 s."""
+    import torch
+
+    class Fake:
+        path = str(tmp_path / "tuning.json")
+        set = []
+        timed = 0
+
+    f = Fake()
+    f.set = []
+
+    def timed(fn, reps=3):
+        f.timed += 1
+        return 1.0
+
+    monkeypatch.setattr(autotune.tvmc, "set_tuning", lambda k, v: f.set.append((k, v)))
+    monkeypatch.setattr(autotune, "_time", timed)
+    monkeypatch.setattr(autotune, "_device_name", lambda: "gpu")
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: torch.zeros(1))
+    lib = tmp_path / "lib.so"
+    lib.write_bytes(b"one build")
+    monkeypatch.setattr(autotune.tvmc, "LIB_PATH", str(lib))
+    f.lib = lib
+    autotune._build.cache_clear()
+    yield f
+    autotune._build.cache_clear()
+
+
+def tune(f, **kw):
+    f.set.clear()
+    f.timed = 0
+    return autotune.tune_commit(0, path=f.path, **SHAPE, **kw)
+
+
+def test_a_choice_is_kept_for_the_same_build_only(fake):
+    first = tune(fake)
+    assert fake.timed > 0
+    assert tune(fake) == first and fake.timed == 0 and dict(fake.set) == first["knobs"]
+    fake.lib.write_bytes(b"another build")
+    autotune._build.cache_clear()
+    tune(fake)
+    assert fake.timed > 0
+
+
+def test_entries_without_a_build_are_not_applied(fake):
+    old = {"knobs": {"lde_mid_variant": 2}, "seconds": {}}
+    with open(fake.path, "w") as fp:
+        json.dump({"gpu|commit|1048576x379x4": old}, fp)
+    assert tune(fake) != old and fake.timed > 0

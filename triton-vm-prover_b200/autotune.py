@@ -2,7 +2,8 @@
 
 Times candidate values of the library's tuning knobs (tvmc_set_tuning) on the
 caller's own table shapes, keeps the fastest, and persists the choice in a JSON
-cache keyed by device name and shape, so later processes start tuned:
+cache keyed by device name, build of the library and shape, so later processes
+start tuned (a choice made among another build's kernels is not taken over):
 
     lde_mid_variant     fused LDE middle kernel: per-coset global twiddles (1) or
                         inter-pass twiddles shared across cosets in shared memory (2),
@@ -21,6 +22,8 @@ register allocation), so tuning never affects results.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import time
@@ -37,6 +40,16 @@ def _device_name() -> str:
         return torch.cuda.get_device_name()
     except Exception:
         return "cuda"
+
+
+@functools.lru_cache(maxsize=None)
+def _build() -> str:
+    with open(tvmc.LIB_PATH, "rb") as f:
+        return hashlib.sha256(f.read()).hexdigest()[:16]
+
+
+def _key(kind: str, shape: str) -> str:
+    return f"{_device_name()}|{_build()}|{kind}|{shape}"
 
 
 def load(path: str = CACHE) -> dict:
@@ -87,7 +100,7 @@ def tune_commit(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, 
     the LDE knobs on the LDE alone (up to 64 of its columns), then the tree
     fusion on whole commits."""
     import torch
-    key = f"{_device_name()}|commit|{trace_len}x{width}x{expansion}"
+    key = _key("commit", f"{trace_len}x{width}x{expansion}")
     db = load(path)
     if key in db and not force:
         apply(db[key]["knobs"])
@@ -128,7 +141,7 @@ def tune_commit(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, 
 
 def tune_batch(shapes, fill, path: str = CACHE, force: bool = False, candidates=(1, 2, 4, 8, 16)) -> dict:
     """Tune batch_streams for a tvmc.Batch of `shapes`; fill(batch) loads inputs."""
-    key = f"{_device_name()}|batch|" + ",".join(f"{s[0]}x{s[1]}" for s in shapes)
+    key = _key("batch", ",".join(f"{s[0]}x{s[1]}" for s in shapes))
     db = load(path)
     if key in db and not force:
         apply(db[key]["knobs"])
@@ -152,7 +165,7 @@ def tune_batch(shapes, fill, path: str = CACHE, force: bool = False, candidates=
 
 def tune_frugal(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, offset: int = 7,
                 path: str = CACHE, force: bool = False, candidates=(10, 20, 40, 80)) -> dict:
-    key = f"{_device_name()}|frugal|{trace_len}x{width}x{expansion}"
+    key = _key("frugal", f"{trace_len}x{width}x{expansion}")
     db = load(path)
     if key in db and not force:
         apply(db[key]["knobs"])
