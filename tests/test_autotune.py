@@ -60,3 +60,9 @@ def test_entries_without_a_build_are_not_applied(fake):
     with open(fake.path, "w") as fp:
         json.dump({"gpu|commit|1048576x379x4": old}, fp)
     assert tune(fake) != old and fake.timed > 0
+
+
+def test_only_knobs_that_do_something_are_timed(fake):
+    entry = tune(fake)
+    assert set(entry["knobs"]) == {"lde_mid_variant", "lde_mid_ctas", "lde_split_l1", "ntt_tile_log"}
+    assert "hash_unfused_tree" not in dict(fake.set)

@@ -12,7 +12,6 @@ start tuned (a choice made among another build's kernels is not taken over):
     lde_split_l1        the LDE's four-step split N = n1 * n2 (balanced, or n1 = N^(1/2) / 4,
                         or n1 = 2^12 where valid)
     ntt_tile_log        words an NTT pass CTA moves per tile (2^12 .. 2^14)
-    hash_unfused_tree   1 = build all Merkle levels in the tree kernel (0, 1)
     batch_streams       worker streams of a tvmc_batch (1 .. 16)
     batch_multi_hash    one multi-table row-hash launch for a batch (1) or per-table hashes (2)
     frugal_stripe_cols  columns per frugal stripe (multiples of 10)
@@ -96,9 +95,8 @@ def lde_candidates(log_n: int):
 
 def tune_commit(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, offset: int = 7,
                 stream=None, path: str = CACHE, force: bool = False) -> dict:
-    """Tune the plain commit of one device-resident column-major table: first
-    the LDE knobs on the LDE alone (up to 64 of its columns), then the tree
-    fusion on whole commits."""
+    """Tune the plain commit of one device-resident column-major table: the LDE
+    knobs, on the LDE alone (up to 64 of its columns)."""
     import torch
     key = _key("commit", f"{trace_len}x{width}x{expansion}")
     db = load(path)
@@ -117,22 +115,7 @@ def tune_commit(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, 
     del out
     best_lde = dict(zip(("lde_mid_variant", "lde_mid_ctas", "lde_split_l1", "ntt_tile_log"),
                         min(lde_s, key=lde_s.get)))
-    apply(best_lde)
-
-    def run():
-        c = tvmc.Commitment(trace_ptr, width=width, trace_len=trace_len, device_ptr=True,
-                            expansion=expansion, offset=offset, stream=stream)
-        c.sync()
-        c.free()
-
-    hash_s = {}
-    for unfused in (0, 1):
-        tvmc.set_tuning("hash_unfused_tree", unfused)
-        hash_s[unfused] = _time(run)
-    best_unfused = min(hash_s, key=hash_s.get)
-    entry = {"knobs": dict(best_lde, hash_unfused_tree=best_unfused),
-             "seconds": {"lde": {",".join(map(str, k)): v for k, v in lde_s.items()},
-                         "commit_by_unfused_tree": {str(k): v for k, v in hash_s.items()}}}
+    entry = {"knobs": best_lde, "seconds": {"lde": {",".join(map(str, k)): v for k, v in lde_s.items()}}}
     apply(entry["knobs"])
     db[key] = entry
     save(db, path)
