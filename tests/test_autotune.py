@@ -66,3 +66,20 @@ def test_only_knobs_that_do_something_are_timed(fake):
     entry = tune(fake)
     assert set(entry["knobs"]) == {"lde_mid_variant", "lde_mid_ctas", "lde_split_l1", "ntt_tile_log"}
     assert "hash_unfused_tree" not in dict(fake.set)
+
+
+@pytest.mark.parametrize("log_n", [8, 12, 13, 16, 17, 20, 22])
+def test_candidates_are_valid_and_distinct(log_n):
+    c = autotune.lde_candidates(log_n)
+    balanced = (log_n + 1) // 2
+    assert len({tuple(x.items()) for x in c}) == len(c)
+    for x in c:
+        s = x["lde_split_l1"]
+        assert s == 0 or (6 <= s <= 12 and 6 <= log_n - s <= 12)
+        if x["lde_mid_variant"] == 0:
+            assert x["lde_mid_ctas"] == 3
+        else:
+            assert s != balanced  # the networks' default
+    if log_n >= 12:
+        assert any(x["lde_mid_variant"] == 0 and x["lde_split_l1"] == balanced for x in c)
+    assert {x["lde_mid_variant"] for x in c if x["lde_split_l1"] == 0} == {0, 1, 2}

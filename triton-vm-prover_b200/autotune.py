@@ -9,8 +9,8 @@ start tuned (a choice made among another build's kernels is not taken over):
                         inter-pass twiddles shared across cosets in shared memory (2),
                         or 2^8- and 2^10-point passes on the tensor cores (0)
     lde_mid_ctas        its resident CTAs/SM (2, 3)
-    lde_split_l1        the LDE's four-step split N = n1 * n2 (balanced, or n1 = N^(1/2) / 4,
-                        or n1 = 2^12 where valid)
+    lde_split_l1        the LDE's four-step split N = n1 * n2 (the default, balanced,
+                        n1 = N^(1/2) / 4, or n1 = 2^12 where valid)
     ntt_tile_log        words an NTT pass CTA moves per tile (2^12 .. 2^14)
     batch_streams       worker streams of a tvmc_batch (1 .. 16)
     batch_multi_hash    one multi-table row-hash launch for a batch (1) or per-table hashes (2)
@@ -87,10 +87,17 @@ def _time(fn, reps: int = 3) -> float:
 
 def lde_candidates(log_n: int):
     """The LDE knob combinations worth timing for a trace of 2^log_n rows."""
-    splits = [0] + [l1 for l1 in (log_n // 2 - 2, 12) if 6 <= l1 <= 12 and 6 <= log_n - l1 <= 12
-                    and l1 != (log_n + 1) // 2]
-    return [{"lde_mid_variant": v, "lde_mid_ctas": c, "lde_split_l1": s, "ntt_tile_log": t}
-            for v in (0, 1, 2) for c in (2, 3) for s in splits for t in (12, 13, 14)]
+    balanced = (log_n + 1) // 2
+    splits = [l1 for l1 in dict.fromkeys((balanced, log_n // 2 - 2, 12)) if 6 <= l1 <= 12 and 6 <= log_n - l1 <= 12]
+
+    def combine(variants, ctas, splits):
+        return [{"lde_mid_variant": v, "lde_mid_ctas": c, "lde_split_l1": s, "ntt_tile_log": t}
+                for v in variants for c in ctas for s in splits for t in (12, 13, 14)]
+
+    # On the tensor cores (variant 0) the default split is the library's own choice,
+    # so the balanced one is a candidate beside it; K2 takes one CTA per SM there.
+    # The register networks' default split is the balanced one.
+    return combine((0,), (3,), [0] + splits) + combine((1, 2), (2, 3), [0] + [s for s in splits if s != balanced])
 
 
 def tune_commit(trace_ptr: int, trace_len: int, width: int, expansion: int = 4, offset: int = 7,
