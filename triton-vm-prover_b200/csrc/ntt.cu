@@ -617,9 +617,11 @@ static int fit_lT(int lT, int ls, int nbuf, int extra = 0) {
 // 57 | 62, x 64 123 | 91, 2^15 x 16 73 | 76, x 64 201 | 173, 2^16 x 4 55 | 72, x 16 116 | 90,
 // 2^17 x 1 90 | 49, 2^18 x 1 98 | 71, 2^20 x 1 150 | 151, x 64 6080 | 4298; inverse NTT of
 // 2^14 x 64 34 | 36, x 256 92 | 79, 2^16 x 16 36 | 34, x 256 288 | 199, 2^18 x 4 34 | 42, x 16
-// 101 | 84, 2^20 x 1 44 | 57, x 4 106 | 104.
+// 101 | 84, 2^20 x 1 44 | 57, x 4 106 | 104.  An NTT of 2^22 points, whose splits
+// leave one of its passes to networks of 2^11 or 2^12 points, does not gain: x 1
+// 124 | 131, x 4 428 | 454, x 16 1665 | 1705; beyond it no pass has a tensor-core size.
 static bool lde_mma_pays(int l, uint64_t cols) { return l >= 17 || (cols << l) >= 1ull << 20; }
-static bool ntt_mma_pays(int l, uint64_t cols) { return (cols << l) >= 3ull << 20; }
+static bool ntt_mma_pays(int l, uint64_t cols) { return l < 22 && (cols << l) >= 3ull << 20; }
 // log2 of the four-step factor n1 that gives the tensor cores the most of a
 // 2^l-point transform: both passes where that is possible, else K2 (n1), the
 // largest part of an LDE.
@@ -715,10 +717,10 @@ cudaError_t launch_lde(const LdePlan& pl, const uint64_t* trace, uint64_t tld, u
         return launch_lde_small(pl, trace, tld, out, old, cols, add, rm, st);
     }
     // four-step split N = n1 * n2 (K2 runs the n1-point transforms, K1 and K3
-    // the n2-point ones); the default is the balanced split, the tuning knob
-    // "lde_split_l1" picks another valid one
-    // (both factors at least 2^6, so that every pass kernel has at least one
-    // whole tile of sequences)
+    // the n2-point ones): the tensor cores' (mma_split) or the balanced one, unless
+    // the tuning knob "lde_split_l1" picks another, with both factors at least 2^6 so
+    // that a tile of the register networks is never short of sequences (mma_split
+    // goes down to n2 = 2^4, where n1 = 2^8 fills the tile)
     const bool mma = tuning_lde_mid_variant() == 3 && lde_mma_pays(l, cols);
     int l1 = mma ? mma_split(l) : (l + 1) / 2;
     if (const int ks = tuning_lde_split_l1(); ks >= 6 && ks <= 12 && l - ks >= 6 && l - ks <= 12) l1 = ks;
