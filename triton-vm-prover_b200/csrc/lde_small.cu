@@ -1,4 +1,6 @@
 // LDE of short columns (N <= 2^11): whole columns per CTA.
+#include <algorithm>
+
 #include "ntt_sub.cuh"
 
 namespace tvmc {
@@ -7,15 +9,18 @@ namespace tvmc {
 // transforms of 2^lc cosets of every column at a time (sequence u = t * 2^lc + c),
 // so that a short column's cosets fill the CTA together and an output row of
 // cosets is written as one run.  One coset at a time left three quarters of the
-// threads idle: 2^8 x 379, x4, 43 -> 26 us.
-template <int LS>
+// threads idle: 2^8 x 379, x4, 43 -> 26 us.  ONE: no expansion, le = lc = 0, where
+// the index arithmetic of cosets is dead weight (2^8 x 379 14.5 us with it, 12.5
+// without; 2^10 x 379 74 and 71).
+template <int LS, bool ONE>
 __global__ void __launch_bounds__(NTT_THREADS) k_lde_small(const uint64_t* trace, uint64_t tld, uint64_t* out,
-                                                           uint64_t old, uint64_t cols, int lT, int le, int lc,
-                                                           const uint64_t* tw12_f, const uint64_t* sc_lo,
+                                                           uint64_t old, uint64_t cols, int lT, int le_arg,
+                                                           int lc_arg, const uint64_t* tw12_f, const uint64_t* sc_lo,
                                                            const uint64_t* sc_hi, int hi_len, const uint64_t* add,
                                                            int rm) {
     extern __shared__ uint64_t sm[];
     constexpr int n = 1 << LS;
+    const int le = ONE ? 0 : le_arg, lc = ONE ? 0 : lc_arg;
     const int E = 1 << le, EC = 1 << lc;
     uint64_t* twf = sm;                    // forward root only (the inverse negates its input index)
     uint64_t* cf = twf + n;                // coefficients (natural order)
@@ -49,15 +54,16 @@ cudaError_t launch_lde_small(const LdePlan& pl, const uint64_t* trace, uint64_t 
                              uint64_t cols, const uint64_t* add, int rm, cudaStream_t st) {
     const int l = pl.logn, le = pl.log_exp;
     const int hi_len = l > 12 ? (1 << (l - 12)) : 1;
-    const int lT = l <= 5 ? (10 - l < 8 ? 10 - l : 8) : (10 - l > 3 ? 3 : (10 - l > 0 ? 10 - l : 0));
+    const int lT = std::clamp(10 - l, 0, l <= 5 ? 8 : 3);  // about 2^10 words of coefficients per CTA
     const int lc = le < 2 ? le : 2;  // four cosets at a time: 100 KB at 2^11
     const int T = 1 << lT;
     const size_t smem = words_bytes((size_t)(1u << l) + spad_words(1 << l, lT) + spad_words(1 << l, lT + lc));
     return dispatch_ls(l, [&]<int LS>() -> cudaError_t {
-        cudaError_t e = set_smem((const void*)k_lde_small<LS>, smem);
+        auto kern = le ? k_lde_small<LS, false> : k_lde_small<LS, true>;
+        cudaError_t e = set_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
         count_launch();
-        k_lde_small<LS><<<(unsigned)((cols + T - 1) / T), NTT_THREADS, smem, st>>>(
+        kern<<<(unsigned)((cols + T - 1) / T), NTT_THREADS, smem, st>>>(
             trace, tld, out, old, cols, lT, le, lc, pl.tw12_f, pl.sc_lo, pl.sc_hi, hi_len, add, rm);
         return cudaGetLastError();
     });
