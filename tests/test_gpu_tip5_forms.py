@@ -37,6 +37,21 @@ def test_pairs_and_permutations_of_both_forms(tv, oracle, count):
         assert (perm[i] == oracle.permutation(s[i] % P)).all()
 
 
+@pytest.mark.parametrize("count", [8192, 8193])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_permutations_at_any_word_of_an_array(tv, oracle, count, shift):
+    """The tensor-core form moves pairs of words where the array's alignment allows it."""
+    s = rand_u64(count + shift, (count, 16), hi=2**64 - 1)
+    d = dev_empty(16 * count + 2)
+    d[shift: shift + 16 * count] = to_dev(s).reshape(-1)
+    d[shift + 16 * count:] = 5
+    tv.tip5_permutations_gpu(d.data_ptr() + 8 * shift, count)
+    got = from_dev(d)
+    for i in (0, 1, 127, 128, count - 1):
+        assert (got[shift + 16 * i: shift + 16 * i + 16] == oracle.permutation(s[i] % P)).all()
+    assert (got[shift + 16 * count:] == 5).all()
+
+
 @pytest.mark.parametrize("logn", [16, 17, 18, 19, 20, 21])
 @pytest.mark.parametrize("cols,exp,offset", [(1, 4, 7), (3, 2, 3), (2, 1, 7), (1, 8, 11)])
 def test_lde_with_tensor_core_passes(tv, oracle, logn, cols, exp, offset):
