@@ -113,8 +113,9 @@ def test_commit_full_size_properties(tv, oracle):
         assert (root < P).all()
 
 
-@pytest.mark.parametrize("knob,value", [("hash_unfused_tree", 1), ("lde_mid_ctas", 3)])
-@pytest.mark.parametrize("logn", [4, 12, 14])
+@pytest.mark.parametrize("knob,value", [("lde_mid_variant", 1), ("lde_mid_variant", 2), ("lde_mid_ctas", 2),
+                                        ("hash_unfused_tree", 1)])
+@pytest.mark.parametrize("logn", [4, 12, 14, 16])  # 2^16 x 23: the default runs on the tensor cores
 def test_tuning_knobs_do_not_change_results(tv, oracle, knob, value, logn):
     """Scheduling knobs change no bit: plain and frugal commits vs the default."""
     t = rand_u64(0xC0FFEE + logn, (23, 1 << logn))

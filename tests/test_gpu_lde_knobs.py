@@ -8,7 +8,7 @@ import itertools
 import numpy as np
 import pytest
 
-from conftest import dev_empty, from_dev, rand_u64, to_dev
+from conftest import P, dev_empty, from_dev, rand_u64, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -40,6 +40,21 @@ def test_lde_every_knob_combination_equals_oracle(knobs, oracle, logn, expansion
         _set(tv, variant, ctas, split, tile)
         got = tv.lde(t, expansion=expansion)
         assert (got == exp).all(), (variant, ctas, split, tile)
+
+
+@pytest.mark.parametrize("logn,cols,expansion", [(12, 256, 2), (14, 64, 4), (16, 16, 8), (17, 1, 16), (18, 2, 4),
+                                                 (20, 1, 4)])
+def test_lde_on_tensor_cores_with_explicit_splits_equals_oracle(knobs, oracle, logn, cols, expansion):
+    """Splits that put all, some or none of the passes on the tensor cores, and the tile
+    sizes of those left on the register networks."""
+    tv = knobs
+    t = rand_u64(7400 + logn, (cols, 1 << logn), hi=2**64 - 1)
+    some = sorted({0, cols // 2, cols - 1})
+    exp = oracle.lde(t[some] % P, expansion=expansion)
+    splits = [0] + [s for s in range(6, 13) if 6 <= logn - s <= 12]
+    for split, tile in itertools.product(splits, (12, 13, 14)):
+        _set(tv, 0, 3, split, tile)
+        assert (tv.lde(t, expansion=expansion)[some] == exp).all(), (split, tile)
 
 
 def test_lde_largest_trace_at_expansion_16(tv, oracle):

@@ -60,6 +60,19 @@ def test_lde_with_tensor_core_passes(tv, oracle, logn, cols, exp, offset):
     assert (tv.lde(t, exp, offset) == oracle.lde(t, exp, offset)).all()
 
 
+@pytest.mark.parametrize("logn,cols,exp", [(12, 256, 4), (13, 128, 2), (14, 64, 4), (15, 32, 8), (16, 16, 1), (16, 37, 16),
+                                           (17, 1, 16), (18, 2, 2), (20, 1, 4), (22, 1, 4)])
+def test_lde_of_any_representatives_where_the_tensor_cores_pay(tv, oracle, logn, cols, exp):
+    """The shortest columns and fewest of them that take these passes, the 10 + 12 split
+    of 2^22 and K2 with sixteen cosets; inputs that are not canonical."""
+    t = rand_u64(logn * 9 + cols, (cols, 1 << logn), hi=2**64 - 1)
+    t[0, : EDGE_VALUES.size] = EDGE_VALUES
+    t[-1, -3:] = [2**64 - 1, P, P + 1]
+    got = tv.lde(t, exp, 7)
+    for c in sorted({0, cols // 2, cols - 1}):
+        assert (got[c] == oracle.lde(t[c: c + 1] % P, exp, 7)[0]).all()
+
+
 def test_lde_column_count_beyond_one_unit(tv, oracle):
     """More columns than one unit of the tensor-core passes holds, and an odd count."""
     t = rand_u64(99, (37, 1 << 20))
@@ -84,7 +97,7 @@ def test_short_columns_with_any_number_of_cosets(tv, oracle, logn, cols, exp):
     assert (tv.lde(t, exp, 7) == oracle.lde(t, exp, 7)).all()
 
 
-@pytest.mark.parametrize("logn,cols", [(12, 800), (13, 400), (16, 48), (18, 13), (20, 3), (21, 2)])
+@pytest.mark.parametrize("logn,cols", [(12, 800), (13, 400), (16, 48), (18, 13), (20, 3), (21, 2), (22, 1)])
 @pytest.mark.parametrize("inverse", [False, True])
 def test_ntt_with_tensor_core_passes(tv, oracle, logn, cols, inverse):
     a = rand_u64(logn + cols, (cols, 1 << logn), hi=2**64 - 1)
