@@ -14,8 +14,9 @@ back); `roofline` = the dominant kernel (Tip5 row hash + tree) against the SM
 instruction-issue limit (SMs x 4 schedulers x 32 lanes x the SM clock sampled
 during the timed region); `roofline_lde` = the LDE kernels against HBM;
 `roofline_commit` = the whole step against the slower of its HBM bytes at the
-measured copy bandwidth and its integer ops (Tip5 + NTT cost model) at the
-issue limit; `cpu_baseline` = the reference's own CPU code (oracle/_ref) on a
+measured copy bandwidth and the instructions its kernels issue at the issue
+limit (both also carry the cost model's operation counts, which are of the
+algorithm without tensor cores); `cpu_baseline` = the reference's own CPU code (oracle/_ref) on a
 bounded sample on this host's cores, extrapolated to the workload.
 
 `--impl reference` times the reference's own CPU code (oracle/_ref, OpenMP on
@@ -62,6 +63,12 @@ METRIC = "committed LDE cells/s"
 OPS_PER_PERM = 5 * (12 * 4 * 16 + 4 * 48 + 640 + 16 * 4)
 # NTT cost model: 24 int32 ops per butterfly or scale.
 OPS_PER_NTT_MUL = 24
+# What the kernels issue (thread-instructions, ncu smsp__inst_executed x 32): per Tip5
+# permutation of a 2^18 x 379 row hash, and per element and transform of a 16 x 2^20
+# LDE onto four cosets (five transforms).  Fewer than the cost models count, since
+# the tensor cores take the MDS and the DFTs.
+INSTR_PER_PERM = 6421
+INSTR_PER_NTT_ELEMENT = 198
 # Instruction issue of one SM per clock: 4 schedulers x 32 lanes.
 ISSUE_LANES_PER_SM = 4 * 32
 
@@ -527,8 +534,8 @@ def run_ours(args):
     hash_ms = [p[2] for p in phases]
     lde_ms = [p[1] for p in phases]
     widths = [W_MAIN, W_AUX] * args.steps
-    ops = [perms_per_table(L, w) * OPS_PER_PERM for w in widths]
-    achieved_int = sum(ops) / (sum(hash_ms) / 1e3) / 1e12
+    perms = sum(perms_per_table(L, w) for w in widths)
+    achieved_int = perms * INSTR_PER_PERM / (sum(hash_ms) / 1e3) / 1e12
     lde_bytes = [8 * n * w + 8 * L * w for w in widths]
     achieved_hbm = sum(lde_bytes) / (sum(lde_ms) / 1e3) / 1e9
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -541,22 +548,26 @@ def run_ours(args):
     int_peak = issue_limit_tops(sms, sm_mhz)
     # whole step: the slower of its HBM bytes and its integer work
     step_bytes = sum(bytes_per_table(n, w) for w in (W_MAIN, W_AUX))
-    step_int_ops = sum(perms_per_table(L, w) * OPS_PER_PERM + ntt_ops_per_table(n, w) for w in (W_MAIN, W_AUX))
+    model_ops = sum(perms_per_table(L, w) * OPS_PER_PERM + ntt_ops_per_table(n, w) for w in (W_MAIN, W_AUX))
+    step_instr = sum(perms_per_table(L, w) * INSTR_PER_PERM + w * (n + L) * INSTR_PER_NTT_ELEMENT
+                     for w in (W_MAIN, W_AUX))
     hbm_ms = step_bytes / (hbm_peak * 1e9) * 1e3
-    int_ms = step_int_ops / (int_peak * 1e12) * 1e3
+    int_ms = step_instr / (int_peak * 1e12) * 1e3
     ms_step = t_max / args.steps
     roof_commit = {"bound": "int32" if int_ms >= hbm_ms else "hbm", "roofline_ms_per_step": max(hbm_ms, int_ms),
                    "ms_per_step": ms_step, "frac": max(hbm_ms, int_ms) / ms_step,
                    "hbm_ms": hbm_ms, "int_ms": int_ms, "bytes_per_step": step_bytes,
-                   "int_ops_per_step": step_int_ops, "hbm_peak_gbs": hbm_peak, "hbm_peak_source": hbm_src,
+                   "instructions_per_step": step_instr, "cost_model_ops_per_step": model_ops, "hbm_peak_gbs": hbm_peak, "hbm_peak_source": hbm_src,
                    "int_peak_tops": int_peak,
+                   "instructions": f"{INSTR_PER_PERM} per Tip5 permutation, {INSTR_PER_NTT_ELEMENT} per element and "
+                                   "transform (ncu)",
                    "cost_model": f"Tip5 {OPS_PER_PERM} int32 ops per permutation; NTT {OPS_PER_NTT_MUL} per "
                                  "butterfly or scale; bytes 8NW + 32NW + 40*4N + 40*(4N-1) per table"}
-    # DRAM bytes per k_hash_rows launch: one ncu capture of the 2^18-row x 379-column
-    # main-table launch (795.6 MB read + 16.0 MB written), scaled by rows
+    # DRAM bytes per k_hash_rows_mma launch: one ncu capture of a 2^18-row x
+    # 379-column launch (798.9 MB read + 21.0 MB written), scaled by rows
     traffic, traffic_src = None, None
     if W_MAIN == 379:
-        traffic = (795.59e6 + 16.05e6) * L / (1 << 18)
+        traffic = (798.92e6 + 21.04e6) * L / (1 << 18)
         traffic_src = "ncu dram__bytes_read+write of a 2^18x379 launch, scaled by LDE rows (main table)"
 
     # e2e: pinned host traces through the public C ABI, roots read back
@@ -668,13 +679,14 @@ def run_ours(args):
                        "tuning": tuned.get("knobs", {}), "tuning_s": tuned.get("seconds", {}),
                        "streams": args.streams,
                        "parallelism": "replicas" if ws > 1 else "1 gpu"},
-            "roofline": {"bound": "int32", "kernel": "k_hash_rows_mma + k_merkle_level_mma + k_merkle_coop (Tip5)",
+            "roofline": {"bound": "int32", "instructions_per_permutation": INSTR_PER_PERM, "kernel": "k_hash_rows_mma + k_merkle_level_mma + k_merkle_coop (Tip5)",
                          "achieved": achieved_int, "peak": int_peak, "unit": "Top/s",
                          "frac": achieved_int / int_peak,
                          "peak_source": f"SM issue limit: {sms} SMs x {ISSUE_LANES_PER_SM} lanes x {sm_mhz:.0f} MHz "
                                         "(median SM clock sampled in the timed region)",
                          "traffic": traffic, "traffic_source": traffic_src,
                          "cost_model": f"{OPS_PER_PERM} int32 ops per Tip5 permutation",
+                         "cost_model_tops": perms * OPS_PER_PERM / (sum(hash_ms) / 1e3) / 1e12,
                          "ms_per_step": sum(hash_ms) / args.steps,
                          "ms_per_table_min_max": [min(hash_ms), max(hash_ms)]},
             "roofline_commit": roof_commit,

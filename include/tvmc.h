@@ -226,7 +226,8 @@ typedef struct tvmc_commitment tvmc_commitment;
  *                         memory for all cosets; default 0: LDE passes of 2^8 and 2^10 points
  *                         run on the tensor cores, others as 2
  *   "lde_split_l1"        log2 of the LDE's four-step factor n1 (6 .. 12, with log2(N) - n1 also
- *                         in 6 .. 12, else the balanced split is used); default 0 = balanced
+ *                         in 6 .. 12, else the default is used); default 0: 2^8 or 2^10 where the
+ *                         tensor cores are used, else balanced
  *   "ntt_tile_log"        log2 of the words an NTT/LDE pass CTA moves per tile (11 .. 15);
  *                         default 0 = 13
  *   "hash_unfused_tree"   accepted and read back; the tree kernels build every Merkle level

@@ -711,9 +711,9 @@ std::atomic<long long> g_tune_unfused_tree{0};
 }  // namespace
 
 std::atomic<long long> g_tune_mid_variant{0};
-// Defaults from an A/B of every combination on 64 columns of 2^20 rows (B200):
-// the table-sharing variant at 3 CTAs/SM was fastest (7.56 ms against 7.71 ms
-// for the per-coset variant and 8.19 ms at 2 CTAs/SM).
+// The default is the tensor-core passes.  Of the register networks' variants the
+// table-sharing one (2) at 3 CTAs/SM is the fastest, on 64 columns of 2^20 rows 7.56
+// ms against 7.71 ms for the per-coset one (1) and 8.19 ms at 2 CTAs/SM.
 int tvmc::tuning_lde_mid_ctas() { return g_tune_mid_ctas.load() == 2 ? 2 : 3; }
 int tvmc::tuning_lde_mid_variant() {
     const long long v = g_tune_mid_variant.load();

@@ -2,7 +2,7 @@
 // small kernels around them.
 //
 // Two forms of the permutation carry the path: the tensor-core form, 128 states
-// per MMA and one per thread (hash_mma.cu), for throughput, and the
+// per MMA with two threads each (hash_mma.cu), for throughput, and the
 // sixteen-lanes-per-state form (hash_coop.cu), for the latency of few states.
 //
 // Merkle: parent = hash_pair(left, right) (src/merkle/merkle_tree.cpp:41-61).
@@ -15,9 +15,11 @@
 namespace tvmc {
 
 // Up to this many rows (of all tables of a launch) the sixteen-lane form is
-// faster.  379 columns: its time grows from 77 us (up to 1024 rows) by 28 us per
-// 1024 rows, while one tile per SM of the tensor-core form takes 318 us however
-// many rows it holds; they meet at about 11000.
+// faster.  379 columns: its time grows from 69 us (up to 1024 rows) by 23 us per
+// 1024 rows, while one tile per SM of the tensor-core form takes 314 us however
+// many rows it holds; they would meet at about 11600.  At 10240 rows, us
+// (sixteen-lane | tensor-core): 9 columns 13.1 | 16.6, 40 41 | 47, 264 199 | 224,
+// 379 277 | 314.
 constexpr uint64_t COOP_MAX_ROWS = 10240;
 // Tree levels with at least this many parents go to the tensor-core form: one
 // level takes it 18-20 us up to 16384 parents; the sixteen-lane form takes 12 us

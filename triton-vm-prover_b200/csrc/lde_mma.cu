@@ -425,7 +425,9 @@ cudaError_t launch(void (*kern)(P...), uint64_t work, uint32_t bytes, cudaStream
 }
 
 // Columns per unit: sixteen, to share a block's tables widely, but fewer (down to
-// one per group) while that leaves fewer than two units per SM.
+// one per group) while that leaves fewer than two units per SM.  Units are dealt
+// whole, so that the busiest CTA can have up to 1.3 times the mean (K1 and K2 of 51
+// columns of 2^20: 1.27; of 379 columns of 2^16: 1.17).
 template <int B>
 uint32_t unit_cols(uint64_t blocks, uint32_t cols) {
     uint32_t unit = 16;

@@ -11,8 +11,8 @@
 // but a second one issued behind the first gets its uploads and launches
 // queued while the first computes, and the stream's cached LDE, scratch and
 // staging buffers pass from one large commit to the next -- so small requests
-// never wait behind large ones and requests of mixed sizes overlap as they
-// arrive.  A host callback
+// do not queue behind large ones: their kernels get in as CTAs of a large commit's
+// kernels end, within about a millisecond each.  A host callback
 // on the stream marks each request done, records its completion time and
 // returns its transient memory to the budget; its Merkle tree (and, with
 // TVMC_SERVER_KEEP_LDE, its LDE) stays on the device for openings until the

@@ -18,13 +18,13 @@
 // more K = 32 step, ones(128 x 32) x their bytes, so they cost no instruction of
 // the threads.
 //
-// What bounds it: the integer pipes, in x^7 (69 instructions a word, whose
-// products and reductions keep both the multiply-add and the ALU pipe about 70%
-// busy) and in the recombination (17 a word).  Against an MDS on the FP64 pipe
+// What bounds it: the integer pipes, in x^7 (69 instructions a word) and in the
+// recombination (17 a word): multiply-add 71% and ALU 64% busy, an instruction
+// issued in 63% of the cycles.  Against an MDS on the FP64 pipe
 // this takes 336 FP64 instructions and the recombination of two 52-bit halves
 // out of a round; what it adds is a shared-memory store of the state, one barrier
 // of the group and the MMA's latency, which the SM's other three groups cover
-// (tensor pipe 15% busy).  Two threads share a state: 64 registers each, 32 warps
+// (tensor pipe 16% busy).  Two threads share a state: 64 registers each, 32 warps
 // per SM.  227328 rows x 379 (three full waves of tiles), B200: the FP64 kernel
 // (one thread per state, six 128-thread CTAs per SM) 2.85 ms; this one 2.40 ms.
 // One thread per state with four or six groups: 2.47 and 2.49; four threads per
