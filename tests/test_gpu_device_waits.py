@@ -96,6 +96,16 @@ def test_batch(tv):
                 b.tables[0].root()
 
 
+def test_batch_before_its_first_run_has_not_failed(tv):
+    """Whatever the tables' memory held before."""
+    with tv.Batch([(64, 3)] * 8) as a:
+        for t in a.tables:
+            memcpy_h2d(t.device_tree(), np.ones(1, dtype=np.uint64))
+    with tv.Batch([(64, 3)] * 8) as b:
+        for t in b.tables:
+            t.sync()
+
+
 def test_server(tv):
     t = rand_u64(2, (COLS, 1 << LOGN))
     with tv.Server() as s:

@@ -1853,6 +1853,7 @@ int tvmc_batch_create(const tvmc_table_shape* shapes, size_t count, tvmc_batch**
             return bail(fail(TVMC_ERR_NOMEM, "cannot allocate table %zu of the batch", i));
         }
         b->inputs.push_back(in);
+        CK(cudaMemset(c->d_nodes, 0, 40));  // the status word, for readers before the first run
         CK(cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming));
         const size_t per = lde_scratch_words(plans[i].logn, plans[i].log_exp, 1) * 8;
         chunk[i] = per ? std::max<size_t>(1, std::min(s.width, budget / per)) : std::max<size_t>(s.width, 1);
